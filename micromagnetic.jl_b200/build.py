@@ -57,12 +57,15 @@ def _stale(src):
     return os.path.getmtime(obj) < max(os.path.getmtime(f) for f in [src] + hdrs)
 
 
-def build(force=False, jobs=4, verbose=False):
+def build(force=False, jobs=os.cpu_count() or 4, verbose=False):
     if not force and not needs_build():
         return LIB
     os.makedirs(OBJ_DIR, exist_ok=True)
     todo = [s for s in sources() if force or verbose or _stale(s)]
     with concurrent.futures.ThreadPoolExecutor(max_workers=jobs) as ex:
+        # the film-column and run-time y passes take longest: first
+        slow = ("mm_rf_c_", "mm_hot_y")
+        todo.sort(key=lambda s: not os.path.basename(s).startswith(slow))
         results = list(ex.map(lambda s: _compile(s, verbose), todo))
     objs = [os.path.join(OBJ_DIR, os.path.basename(s) + ".o") for s in sources()]
     if verbose:
@@ -80,7 +83,7 @@ def build(force=False, jobs=4, verbose=False):
 if __name__ == "__main__":
     ap = argparse.ArgumentParser()
     ap.add_argument("--force", action="store_true")
-    ap.add_argument("-j", type=int, default=4)
+    ap.add_argument("-j", type=int, default=os.cpu_count() or 4)
     ap.add_argument("-v", action="store_true", help="print ptxas resource usage")
     a = ap.parse_args()
     print(build(force=a.force, jobs=a.j, verbose=a.v))

@@ -132,6 +132,7 @@ class Engine : public EngineBase {
     if (dp_graph) cudaGraphExecDestroy(dp_graph);
     if (he_graph) cudaGraphExecDestroy(he_graph);
     demag.reset();
+    demag_sd.reset();
     for (void* p : allocs_) cudaFree(p);
     if (st_) cudaStreamDestroy(st_);
   }
@@ -153,7 +154,9 @@ class Engine : public EngineBase {
   }
 
   cudaStream_t stream() const override { return st_; }
-  size_t device_bytes() const override { return bytes_ + (demag ? demag->device_bytes() : 0); }
+  size_t device_bytes() const override {
+    return bytes_ + (demag ? demag->device_bytes() : 0) + (demag_sd ? demag_sd->device_bytes() : 0);
+  }
 
   // ------------------------------------------------------------ setup --
   int set_Ms(const double* Msh, double uni) override {
@@ -452,12 +455,10 @@ class Engine : public EngineBase {
     return MM_OK;
   }
 
-  int add_demag(int Nx, int Ny, int Nz, const double* T6N_host) override {
-    if (mask & TB_DEMAG) return fail(MM_ERR_UNSUPPORTED, "one demag term per handle");
-    if (Nx < 0 || Ny < 0 || Nz < 0) return fail(MM_ERR_ARG, "macro-PBC image counts must be >= 0");
-    auto plan = std::make_unique<DemagPlan<R>>();
+  // geometry, buffers and tensor spectrum of a plan
+  int build_demag(DemagPlan<R>& plan, int Nx, int Ny, int Nz, const double* T6N_host, bool runtime_len) {
     char msg[256] = {0};
-    int rc = plan->init(nx, ny, nz, st_, msg, sizeof(msg));
+    int rc = plan.init(nx, ny, nz, st_, msg, sizeof(msg), runtime_len);
     if (rc == -1) return fail(MM_ERR_ARG, "%s", msg);
     if (rc) return fail(MM_ERR_CUDA, "demag plan allocation failed (%d)", rc);
     double* T = nullptr;
@@ -468,10 +469,40 @@ class Engine : public EngineBase {
       cudaFree(T);
       return fail(MM_ERR_CUDA, "Newell tensor assembly failed: %s", cudaGetErrorString(static_cast<cudaError_t>(rc)));
     }
-    rc = plan->set_tensor(T, st_);
+    rc = plan.set_tensor(T, st_);
     cudaStreamSynchronize(st_);
     cudaFree(T);
     if (rc) return fail(MM_ERR_CUDA, "demag tensor assembly failed: %s", cudaGetErrorString(static_cast<cudaError_t>(rc)));
+    return MM_OK;
+  }
+
+  // The plan steepest descents of FP64 films use: the run-time-length passes.
+  // The Barzilai-Borwein step lengths amplify rounding (two FFTs that differ by
+  // 1e-16 leave states 1e-8 apart after 60 steps, and the step at which the
+  // stopping criterion is met moves by a third), so a descent keeps the
+  // arithmetic its earlier results came from.  Where the compile-time lengths
+  // differ from the run-time ones the second plan is built at the first
+  // descent.  Nullptr on failure.
+  DemagPlan<R>* sd_plan() {
+    if (!demag || kF32 || nz > 1 || !demag->rfft || demag->runtime_ok) return demag.get();
+    if (!demag_sd) {
+      auto p = std::make_unique<DemagPlan<R>>();
+      if (build_demag(*p, images_[0], images_[1], images_[2], tensor_.empty() ? nullptr : tensor_.data(), true))
+        return nullptr;
+      demag_sd = std::move(p);
+    }
+    return demag_sd.get();
+  }
+
+  int add_demag(int Nx, int Ny, int Nz, const double* T6N_host) override {
+    if (mask & TB_DEMAG) return fail(MM_ERR_UNSUPPORTED, "one demag term per handle");
+    if (Nx < 0 || Ny < 0 || Nz < 0) return fail(MM_ERR_ARG, "macro-PBC image counts must be >= 0");
+    auto plan = std::make_unique<DemagPlan<R>>();
+    if (int rc = build_demag(*plan, Nx, Ny, Nz, T6N_host, false)) return rc;
+    images_[0] = Nx; images_[1] = Ny; images_[2] = Nz;
+    // a tensor of the caller's is kept where a descent may need it again (sd_plan)
+    if (T6N_host && !kF32 && nz == 1 && plan->rfft && !plan->runtime_ok) tensor_.assign(T6N_host, T6N_host + 6 * N);
+    int rc;
     if (!Hd && (rc = alloc(Hd, 3 * N))) return rc;
     // tile widths of the strided passes, timed on this plan's own buffers
     if ((rc = plan->autotune(m, Ms, Hd, st_))) return fail(MM_ERR_CUDA, "demag tile autotuning failed (%d)", rc);
@@ -1100,8 +1131,15 @@ class Engine : public EngineBase {
       SdState hs{0.0, 1.0, 1e-10, sd_steps};
       MM_CUDA(cudaMemcpyAsync(sd, &hs, sizeof(hs), cudaMemcpyHostToDevice, st_));
       const int nb = stage_blocks(N);
+      const bool dm = (mask & TB_DEMAG) && demag;
+      DemagPlan<R>* const plan = dm ? sd_plan() : nullptr;
+      if (dm && !plan) return MM_ERR_CUDA;
       for (; i <= max_steps; ++i) {
-        enqueue_field(m, work, ~0u, nullptr);
+        enqueue_thermal(th_step, nullptr, th_dt, nullptr);
+        if (plan) plan->apply(m, Ms, Hd, st_, nullptr, plan->runtime_ok && !kF32);
+        StageArgs<R> sf{};
+        sf.out = work;
+        launch_stage<R>(SM_FIELD, fargs(~0u), m, sf, st_);
         launch_sd_gk<R>(m, pre, work, gk, N, sd_steps == 0 ? 1 : 0, partials, st_);
         launch_sd_tau(sd, partials, nb, st_);
         launch_sd_update<R>(m, pre, work, gk, pins_on ? pins : nullptr, sd, N, st_);
@@ -1342,7 +1380,9 @@ class Engine : public EngineBase {
   DopriCtrl hctrl{};
   SdState* sd = nullptr;
   long long sd_steps = 0;
-  std::unique_ptr<DemagPlan<R>> demag;
+  std::unique_ptr<DemagPlan<R>> demag, demag_sd;
+  int images_[3] = {0, 0, 0};
+  std::vector<double> tensor_;
   unsigned mask = 0;
   bool ms_set = false, pins_on = false, ex_spatial = false, id_spatial = false, an_spatial = false, hz_arr = false;
   double ex_A[3] = {0, 0, 0}, bd[3] = {0, 0, 0}, id_D = 0, an_K = 0, an_u[3] = {0, 0, 1}, hz_uni[3] = {0, 0, 0};

@@ -13,223 +13,14 @@
 
 #include "mm_dd.cuh"
 #include "mm_demag.cuh"
+#include "mm_hotpass.cuh"
+#include "mm_persist.cuh"
 #include "mm_passes.cuh"
 #include "mm_fft.cuh"
 #include "mm_launch.cuh"
 #include "mm_lines.cuh"
 
 namespace mm {
-
-static int floor_pow2(int v) {
-  int p = 1;
-  while (p * 2 <= v) p *= 2;
-  return p;
-}
-static int ilog2(int v) {
-  int l = 0;
-  while ((1 << l) < v) ++l;
-  return l;
-}
-
-// Shared-memory budget of one strided-pass block; the kx tile W is the
-// largest power of two (up to 128 bytes of row segment) that fits.
-// Multiprocessors of the current device (cached on first use)
-static int sm_count() {
-  static const int v = [] {
-    int dev = 0, n = 0;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev);
-    return n > 0 ? n : 148;
-  }();
-  return v;
-}
-
-// Lines a shared-memory x-pass block transforms: as many as fill its tile
-// (cap / Lc), but for a mesh launched alone no more than spread `lines` over
-// two blocks an SM -- on small meshes (c1: 150 lines of 200 points) more,
-// shorter blocks finish sooner than a few full ones.  A pass recorded for a
-// batch keeps full tiles: its launch covers the lines of every mesh.  Each
-// line's arithmetic is the same whatever block it lands in.
-template <typename R, int NT>
-static int x_lines_per_block(int lines, int Lc) {
-  const int full = std::max(1, PassCfg<R, NT>::cap / Lc);
-  if (launch_recorder()) return full;
-  const int spread = std::max(1, (lines + 2 * sm_count() - 1) / (2 * sm_count()));
-  return std::min(full, spread);
-}
-
-static int smem_budget_bytes() {
-  static int v = [] {
-    const char* e = getenv("MMCUDA_LINES_SMEM_KB");
-    const int kb = e ? atoi(e) : 100;
-    return (kb > 8 && kb <= 200 ? kb : 100) * 1024;
-  }();
-  return v;
-}
-
-
-// Largest power-of-two radix of the FP32 shared-memory passes (32 or 16;
-// MMCUDA_MAXRADIX=16 selects 16).  A radix-32 butterfly holds 32 complex
-// values a thread, a little above the 80-register budget of the
-// 3-blocks-per-SM passes (a few spilled words), yet one stage fewer a line:
-// c2's 512-point FP32 y passes take 0.076 ms with radix 32 and 0.114 ms with
-// radix 16.
-static int fp32_max_radix() {
-  static const int v = [] {
-    const char* e = getenv("MMCUDA_MAXRADIX");
-    return e && atoi(e) == 16 ? 16 : 32;
-  }();
-  return v;
-}
-
-// The register-resident x and y passes (mm_wreg.cu) where they apply, unless
-// MMCUDA_WREG=0 keeps the shared-memory kernels
-static bool wreg_enabled() {
-  static const bool on = [] {
-    const char* e = getenv("MMCUDA_WREG");
-    return !(e && e[0] == '0');
-  }();
-  return on;
-}
-
-// The direct-DFT z convolution for Pz <= 9 (ZSmall) unless MMCUDA_ZSMALL=0
-static bool zsmall_enabled() {
-  static const bool on = [] {
-    const char* e = getenv("MMCUDA_ZSMALL");
-    return !(e && e[0] == '0');
-  }();
-  return on;
-}
-
-// The register-resident z convolution (mm_zpair.cu) where it applies, unless
-// MMCUDA_ZPAIR=0 keeps the shared-memory kernels
-static bool zpair_enabled() {
-  static const bool on = [] {
-    const char* e = getenv("MMCUDA_ZPAIR");
-    return !(e && e[0] == '0');
-  }();
-  return on;
-}
-
-// 3-D column-major spectra (DemagGeom::yT) unless MMCUDA_COLS3D=0 keeps the
-// row-major layout; both run the same arithmetic on every line
-static bool cols3d_enabled() {
-  static const bool on = [] {
-    const char* e = getenv("MMCUDA_COLS3D");
-    return !(e && e[0] == '0');
-  }();
-  return on;
-}
-
-// z convolution for Pz = RA * RB (powers of two): forward radix-RA stage from
-// the Y rows into shared memory; then, per butterfly i < RA and in registers,
-// the forward radix-RB stage (outputs kz = i + r*RA), the tensor product at
-// those kz for the three components, and the inverse radix-RB stage (its
-// inputs are the same positions), written back in place after a barrier;
-// finally the inverse radix-RA stage straight to the Y rows kz < nz.
-// One shared buffer; requires W * RA <= NT (one middle task per thread).
-// YT (column-major spectra, DemagGeom::yT): a block takes one kx and a tile of
-// W consecutive ky (grid: (Hx, ky tiles), tile q and its mirror Py/W-1-q
-// adjacent in launch order); the tile's rows are W contiguous entries of
-// Y[((c*Hx + kx)*nz + z)*Py + ky], the tensor Nhat[((c*Tzq + kz)*Hx + kx)*Tyq + ky].
-// Row-major: blocks blockIdx.x < nfull take W-wide kx tiles; the columns
-// kx >= nfull * W left over (Hx = 16 m + 1 for nx = 2^k) are tiled along ky
-// instead, block (nfull + r, q) taking column nfull * W + r and ky in
-// [q W, q W + W) (the blocks with q W >= Py return), so that no block
-// transforms a tile of mostly absent columns.
-template <typename R, int RA, int RB, int NT, bool I32, bool YT = false>
-__global__ void __launch_bounds__(NT, (zconv2_minb<R, NT>())) k_zconv2(cplx_t<R>* Y, const R* __restrict__ Nhat, DemagGeom g, int lgW,
-                                                  FastDiv fnl, const cplx_t<R>* __restrict__ twz, int nfull) {
-  using C = cplx_t<R>;
-  using IX = std::conditional_t<I32, int, int64_t>;
-  constexpr int L = RA * RB;
-  extern __shared__ __align__(16) unsigned char smem_raw[];
-  C* a = reinterpret_cast<C*>(smem_raw);
-  pdl_enter();
-  if (g.gate && !*g.gate) return;
-  const int LS = L | 1, Hx = g.Hx, Py = g.Py, nz = g.nz;
-  const int W = 1 << lgW;
-  const int bq = blockIdx.y;
-  int kx0, ky0;  // first column of the tile: (kx0 + w, ky0) or, along ky, (kx0, ky0 + w)
-  bool along_ky = YT;
-  if (YT) {
-    const int nq = gridDim.y;
-    kx0 = blockIdx.x;
-    ky0 = ((bq & 1) ? nq - 1 - (bq >> 1) : (bq >> 1)) << lgW;
-  } else if (static_cast<int>(blockIdx.x) >= nfull) {
-    if ((bq << lgW) >= Py) return;
-    kx0 = nfull * W + (blockIdx.x - nfull);
-    ky0 = bq << lgW;
-    along_ky = true;
-  } else {
-    const int q = (bq + 1) >> 1;
-    kx0 = blockIdx.x * W;
-    ky0 = bq == 0 ? 0 : ((bq & 1) ? q : Py - q);
-  }
-  const int nlines = 3 * W;
-  // rows of the tile: element (c, z, w) at base + c*cs + z*rs + (t0 + w)*ws, t0 + w < tn
-  const IX cs = static_cast<IX>(static_cast<int64_t>(nz) * Py * Hx), rs = static_cast<IX>(YT ? Py : static_cast<int64_t>(Py) * Hx);
-  C* base = YT ? Y + static_cast<int64_t>(kx0) * nz * Py : (along_ky ? Y + kx0 : Y + static_cast<int64_t>(ky0) * Hx);
-  const int t0 = along_ky ? ky0 : kx0, tn = along_ky ? Py : Hx;
-  const IX ws = static_cast<IX>(along_ky && !YT ? Hx : 1);
-  RowsInW<C, IX> src{base, cs, rs, ws, lgW, t0, tn, nz};
-  RowsOutW<C, IX> dst{base, cs, rs, ws, lgW, t0, tn, nz};
-  SmemLines<C> A{a, LS};
-  lstage<RA, false, true, NT>(src, A, L, nlines, fnl, 1, twz, 1);
-  // fused middle: thread -> (w, i), w fastest
-  const int task = threadIdx.x;
-  const bool act = task < W * RA;
-  const int w = task & (W - 1), i = task >> lgW;
-  const int kx = along_ky ? kx0 : kx0 + w;
-  const int ky = along_ky ? ky0 + w : ky0;
-  C v[3][RB];
-  if (act) {
-#pragma unroll
-    for (int c = 0; c < 3; ++c) {
-#pragma unroll
-      for (int r = 0; r < RB; ++r) v[c][r] = A.load(c * W + w, i + r * RA);
-      // forward radix-RB stage, span p = RA, k = i: twiddles w_L^(r*i)
-#pragma unroll
-      for (int r = 1; r < RB; ++r) v[c][r] = cmul(v[c][r], __ldg(twz + r * i));
-      dftR<RB, false>(v[c]);
-    }
-    if (kx < Hx && ky < Py) {
-      const int Tyq = Py / 2 + 1, Tzq = L / 2 + 1;
-      const int64_t Ts = static_cast<int64_t>(Tzq) * Tyq * Hx;
-      const bool fy = ky > Py / 2;
-      const int kyq = fy ? Py - ky : ky;
-      const R sy = fy ? R(-1) : R(1);
-#pragma unroll
-      for (int r = 0; r < RB; ++r) {
-        const int kz = i + r * RA;
-        const bool fz = kz > L / 2;
-        const int kzq = fz ? L - kz : kz;
-        const R sz = fz ? R(-1) : R(1);
-        const int64_t b = YT ? (static_cast<int64_t>(kzq) * Hx + kx) * Tyq + kyq
-                             : (static_cast<int64_t>(kzq) * Tyq + kyq) * Hx + kx;
-        const R xx = __ldg(Nhat + b), yy = __ldg(Nhat + Ts + b), zz = __ldg(Nhat + 2 * Ts + b);
-        const R xy = sy * __ldg(Nhat + 3 * Ts + b), xz = sz * __ldg(Nhat + 4 * Ts + b),
-                yz = sy * sz * __ldg(Nhat + 5 * Ts + b);
-        const C p0 = v[0][r], p1 = v[1][r], p2 = v[2][r];
-        v[0][r] = cmk<C>(xx * p0.x + xy * p1.x + xz * p2.x, xx * p0.y + xy * p1.y + xz * p2.y);
-        v[1][r] = cmk<C>(xy * p0.x + yy * p1.x + yz * p2.x, xy * p0.y + yy * p1.y + yz * p2.y);
-        v[2][r] = cmk<C>(xz * p0.x + yz * p1.x + zz * p2.x, xz * p0.y + yz * p1.y + zz * p2.y);
-      }
-    }
-    // inverse radix-RB stage, span 1: outputs at i*RB + r
-#pragma unroll
-    for (int c = 0; c < 3; ++c) dftR<RB, true>(v[c]);
-  }
-  __syncthreads();
-  if (act) {
-#pragma unroll
-    for (int c = 0; c < 3; ++c)
-#pragma unroll
-      for (int r = 0; r < RB; ++r) A.store(c * W + w, i * RB + r, v[c][r]);
-  }
-  __syncthreads();
-  lstage<RA, true, true, NT>(A, dst, L, nlines, fnl, RB, twz, 1);
-}
 
 // FP64 tensor quadrant [6][Tzq][Tyq][Hx] to RO, column-major [6][Tzq][Hx][Tys]
 // (rows of Tyq values at stride Tys >= Tyq; films: Tzq = 1)
@@ -489,53 +280,6 @@ static C* upload_twiddles(int L, size_t& bytes, cudaStream_t st) {
   return d;
 }
 
-template <typename R, int NT>
-static void set_smem_attrs_nt() {
-  const int mx = static_cast<int>(kMaxSmem);
-  cudaFuncSetAttribute(k_one<FwdX<R, XM_MAGN, NT>>, cudaFuncAttributeMaxDynamicSharedMemorySize, mx);
-  cudaFuncSetAttribute(k_one<FwdX<R, XM_TENSOR, NT>>, cudaFuncAttributeMaxDynamicSharedMemorySize, mx);
-  cudaFuncSetAttribute(k_one<InvX<R, NT>>, cudaFuncAttributeMaxDynamicSharedMemorySize, mx);
-  cudaFuncSetAttribute(k_ypass<R, YM_FWD, NT>, cudaFuncAttributeMaxDynamicSharedMemorySize, mx);
-  cudaFuncSetAttribute(k_ypass<R, YM_INV, NT>, cudaFuncAttributeMaxDynamicSharedMemorySize, mx);
-  cudaFuncSetAttribute(k_ypass<R, YM_CONV2D, NT>, cudaFuncAttributeMaxDynamicSharedMemorySize, mx);
-  cudaFuncSetAttribute(k_ypass<R, YM_TENSOR, NT>, cudaFuncAttributeMaxDynamicSharedMemorySize, mx);
-  cudaFuncSetAttribute(k_ypass<R, YM_TENSOR_Q, NT>, cudaFuncAttributeMaxDynamicSharedMemorySize, mx);
-  cudaFuncSetAttribute(k_zpass<R, ZM_CONV, NT>, cudaFuncAttributeMaxDynamicSharedMemorySize, mx);
-  cudaFuncSetAttribute(k_zpass<R, ZM_TENSOR_Q, NT>, cudaFuncAttributeMaxDynamicSharedMemorySize, mx);
-  cudaFuncSetAttribute(k_one<YLines<R, YL_FWD, NT, true>>, cudaFuncAttributeMaxDynamicSharedMemorySize, mx);
-  cudaFuncSetAttribute(k_one<YLines<R, YL_INV, NT, true>>, cudaFuncAttributeMaxDynamicSharedMemorySize, mx);
-  cudaFuncSetAttribute(k_one<YLines<R, YL_CONV2D, NT, true>>, cudaFuncAttributeMaxDynamicSharedMemorySize, mx);
-  cudaFuncSetAttribute(k_one<ZConv<R, NT, true>>, cudaFuncAttributeMaxDynamicSharedMemorySize, mx);
-  cudaFuncSetAttribute(k_one<YLines<R, YL_FWD, NT, false>>, cudaFuncAttributeMaxDynamicSharedMemorySize, mx);
-  cudaFuncSetAttribute(k_one<YLines<R, YL_INV, NT, false>>, cudaFuncAttributeMaxDynamicSharedMemorySize, mx);
-  cudaFuncSetAttribute(k_one<YLines<R, YL_CONV2D, NT, false>>, cudaFuncAttributeMaxDynamicSharedMemorySize, mx);
-  cudaFuncSetAttribute(k_one<YLines<R, YL_CONV2D, NT, true, true>>, cudaFuncAttributeMaxDynamicSharedMemorySize, mx);
-  cudaFuncSetAttribute(k_one<YLines<R, YL_CONV2D, NT, false, true>>, cudaFuncAttributeMaxDynamicSharedMemorySize, mx);
-  cudaFuncSetAttribute(k_one<YLines<R, YL_FWD, NT, true, true>>, cudaFuncAttributeMaxDynamicSharedMemorySize, mx);
-  cudaFuncSetAttribute(k_one<YLines<R, YL_FWD, NT, false, true>>, cudaFuncAttributeMaxDynamicSharedMemorySize, mx);
-  cudaFuncSetAttribute(k_one<YLines<R, YL_INV, NT, true, true>>, cudaFuncAttributeMaxDynamicSharedMemorySize, mx);
-  cudaFuncSetAttribute(k_one<YLines<R, YL_INV, NT, false, true>>, cudaFuncAttributeMaxDynamicSharedMemorySize, mx);
-  cudaFuncSetAttribute(k_one<ZConv<R, NT, false>>, cudaFuncAttributeMaxDynamicSharedMemorySize, mx);
-}
-
-template <typename R>
-static void set_smem_attrs() {
-  // one bit per device, set only once the attributes are in place; the lock
-  // keeps a second thread from launching before that (devices >= 64 set the
-  // attributes on every call)
-  static std::mutex mu;
-  static uint64_t done_mask = 0;
-  int dev = 0;
-  cudaGetDevice(&dev);
-  const bool tracked = dev >= 0 && dev < 64;
-  std::lock_guard<std::mutex> lk(mu);
-  if (tracked && ((done_mask >> dev) & 1ull)) return;
-  set_smem_attrs_nt<R, kHotNT>();
-  if (sizeof(R) == 8) set_smem_attrs_nt<double, kTensorNT>();
-  wreg_set_attrs();
-  if (tracked) done_mask |= 1ull << dev;
-}
-
 template <typename R>
 DemagPlan<R>::~DemagPlan() {
   cudaFree(X);
@@ -547,18 +291,70 @@ DemagPlan<R>::~DemagPlan() {
   cudaFree(twx);
   cudaFree(twy);
   cudaFree(twz);
+  cudaFree(rtab);
+}
+
+// The compile-time passes (mm_rf.cuh) where they apply, unless MMCUDA_RFFT=0
+// (or the persistent step kernel, which runs the run-time-length bodies) keeps
+// the run-time-length passes
+static bool rfft_enabled() {
+  static const bool on = [] {
+    const char* e = getenv("MMCUDA_RFFT");
+    return !(e && e[0] == '0');
+  }();
+  return on && !persist_enabled();
+}
+// Smaller meshes keep the run-time-length passes: their kernels are the same
+// for every length, so a batch of them shares launches, and one such mesh is
+// bound by launches either way.
+constexpr int64_t kRfftCells = 8192;
+
+// tw2[(r-1) R1 + k] = w_{R1 R2}^(r k), tw3[(q-1) R1 R2 + i] = w_L^(q i)
+template <typename C>
+static void fill_rf_twiddles(const rf::Radices& f, std::vector<C>& out, size_t& o2, size_t& o3) {
+  const int L = f.r1 * f.r2 * f.r3, M = f.r1 * f.r2;
+  auto push = [&](int64_t num, int den) {
+    const long double a = -2.0L * 3.141592653589793238462643383279502884L * static_cast<long double>(num % den) / den;
+    C c;
+    c.x = static_cast<decltype(C::x)>(static_cast<double>(cosl(a)));
+    c.y = static_cast<decltype(C::x)>(static_cast<double>(sinl(a)));
+    out.push_back(c);
+  };
+  o2 = out.size();
+  for (int r = 1; r < f.r2; ++r)
+    for (int k = 0; k < f.r1; ++k) push(static_cast<int64_t>(r) * k, M);
+  o3 = out.size();
+  for (int q = 1; q < f.r3; ++q)
+    for (int i = 0; i < M; ++i) push(static_cast<int64_t>(q) * i, L);
 }
 
 template <typename R>
-static int lines_tile(int Hx, int L, int lines_per_col, int nbuf);
-
-template <typename R>
-int DemagPlan<R>::init(int nx, int ny, int nz, cudaStream_t st, char* err, size_t nerr) {
+int DemagPlan<R>::init(int nx, int ny, int nz, cudaStream_t st, char* err, size_t nerr, bool runtime_len) {
+  constexpr bool f64 = sizeof(R) == 8;
   g.nx = nx; g.ny = ny; g.nz = nz;
   g.gate = nullptr;
   g.Px = padded_fft_len(nx, true);
   g.Py = padded_fft_len(ny, false);
   g.Pz = padded_fft_len(nz, false);
+  // compile-time lengths: not for the power-of-two meshes of the register
+  // passes (mm_wreg.cu), nor where a line has no instantiation
+  rfft = rfft_z = runtime_ok = false;
+  if (!runtime_len && rfft_enabled() && nx >= 8 && ny >= 8 && static_cast<int64_t>(nx) * ny * nz >= kRfftCells) {
+    const bool zc2 = (g.Pz & (g.Pz - 1)) == 0 && g.Pz >= 4 && (g.Pz <= 128 || (!f64 && g.Pz == 256));
+    const bool reg = nz > 1 && zc2 && wreg_enabled() && wreg_applies(nx, ny, nz, g.Px, g.Py, f64);
+    const int lx = rf::next_length(rf::KX, f64, nx);
+    const int ly = rf::next_length(nz == 1 ? rf::KC : rf::KY, f64, 2 * ny - 1);
+    const int lz = nz >= 6 ? rf::next_length(rf::KZ, f64, 2 * nz - 1) : g.Pz;
+    if (!reg && lx && ly && lz) {
+      rfft = true;
+      runtime_ok = nz == 1 && g.Px == 2 * lx && g.Py == ly &&
+                   6 * sizeof(C) * static_cast<size_t>(padded_line_stride(ly)) <= kMaxSmem;
+      g.Px = 2 * lx;
+      g.Py = ly;
+      g.Pz = lz;
+      rfft_z = nz >= 6 && (f64 || !zpair_enabled() || lz != 32);  // FP32 Pz = 32: register z convolution
+    }
+  }
   g.Lc = g.Px > 1 ? g.Px / 2 : 0;
   g.Hx = g.Px > 1 ? g.Lc + 1 : 1;
   g.Tyq = g.Py / 2 + 1;
@@ -587,6 +383,7 @@ int DemagPlan<R>::init(int nx, int ny, int nz, cudaStream_t st, char* err, size_
   fused2d = !long_y && (g.Pz == 1) &&
             (2 * 3 * (g.Py | 1) * sizeof(C) <= static_cast<size_t>(smem_budget_bytes()) ||
              (cols_ok && 2 * 3 * static_cast<size_t>(padded_line_stride(g.Py)) * sizeof(C) <= kMaxSmem));
+  if (rfft) fused2d = g.Pz == 1;
   if (g.Pz == 1 && !fused2d && cols_ok) long_y = true;
   g.xT = fused2d && cols_ok ? 1 : 0;
   // 3-D meshes whose shared-memory y lines leave row tiles narrower than 8
@@ -594,13 +391,13 @@ int DemagPlan<R>::init(int nx, int ny, int nz, cudaStream_t st, char* err, size_
   // (DemagGeom::yT) when the z convolution is the fused power-of-two kernel
   g.yT = 0;
   const bool zc2 = (g.Pz & (g.Pz - 1)) == 0 && g.Pz >= 4 && (g.Pz <= 128 || (sizeof(R) == 4 && g.Pz == 256));
-  if (g.Pz > 1 && !long_y && cols_ok && zc2 && cols3d_enabled()) {
+  if (g.Pz > 1 && !rfft && !long_y && cols_ok && zc2 && cols3d_enabled()) {
     FftPlan1 py;
     make_fft_plan(g.Py, py, sizeof(R) == 4 ? fp32_max_radix() : 8);
     if (lines_tile<R>(g.Hx, g.Py, 1, std::max(1, line_fft_buffers(py))) < 8) g.yT = g.xT = 1;
   }
   g.wreg = 0;
-  if (g.Pz > 1 && !long_x && !long_y && zc2 && wreg_enabled() &&
+  if (g.Pz > 1 && !rfft && !long_x && !long_y && zc2 && wreg_enabled() &&
       wreg_applies(nx, ny, nz, g.Px, g.Py, sizeof(R) == 8))
     g.wreg = g.yT = g.xT = 1;
   if ((long_x && !make_fft_plan(g.Lc, gplx, 8)) || (long_y && !make_fft_plan(g.Py, gply, 8))) {
@@ -622,8 +419,7 @@ int DemagPlan<R>::init(int nx, int ny, int nz, cudaStream_t st, char* err, size_
   g.frows = make_fastdiv(ny * nz);
   g.fpady = make_fastdiv(std::max(1, g.Py - ny));
   g.fpadz = make_fastdiv(std::max(1, g.Pz - nz));
-  set_smem_attrs<R>();
-  set_smem_attrs<double>();
+  wreg_set_attrs();
   const int64_t nX = 3LL * nz * ny * g.Hx;
   if (cudaMalloc(&X, sizeof(C) * nX) != cudaSuccess) return 2;
   bytes_ += sizeof(C) * nX;
@@ -631,7 +427,7 @@ int DemagPlan<R>::init(int nx, int ny, int nz, cudaStream_t st, char* err, size_
     const int64_t nY = 3LL * nz * g.Py * g.Hx;
     if (cudaMalloc(&Y, sizeof(C) * nY) != cudaSuccess) return 2;
     bytes_ += sizeof(C) * nY;
-    if (long_y) {
+    if (long_y && !rfft) {
       if (cudaMalloc(&S, sizeof(C) * nY) != cudaSuccess) return 2;
       bytes_ += sizeof(C) * nY;
     }
@@ -655,6 +451,20 @@ int DemagPlan<R>::init(int nx, int ny, int nz, cudaStream_t st, char* err, size_
   if (g.Px > 1 && !(twx = upload_twiddles<C>(g.Px, bytes_, st))) return 2;
   if (!(twy = upload_twiddles<C>(g.Py, bytes_, st))) return 2;
   if (!(twz = upload_twiddles<C>(g.Pz, bytes_, st))) return 2;
+  if (rfft) {
+    std::vector<C> h;
+    size_t o[6] = {};
+    fill_rf_twiddles(rf::plan_of(rf::KX, f64, g.Lc), h, o[0], o[1]);
+    fill_rf_twiddles(rf::plan_of(fused2d ? rf::KC : rf::KY, f64, g.Py), h, o[2], o[3]);
+    if (rfft_z) fill_rf_twiddles(rf::plan_of(rf::KZ, f64, g.Pz), h, o[4], o[5]);
+    if (cudaMalloc(&rtab, sizeof(C) * h.size()) != cudaSuccess) return 2;
+    bytes_ += sizeof(C) * h.size();
+    cudaMemcpyAsync(rtab, h.data(), sizeof(C) * h.size(), cudaMemcpyHostToDevice, st);
+    cudaStreamSynchronize(st);
+    rtx = {rtab + o[0], rtab + o[1]};
+    rty = {rtab + o[2], rtab + o[3]};
+    rtz = {rtab + o[4], rtab + o[5]};
+  }
   return static_cast<int>(cudaGetLastError());
 }
 
@@ -909,23 +719,6 @@ __global__ void k_gx_unpack(const cplx_t<R>* __restrict__ Z, R* __restrict__ H, 
 
 // ---- launch helpers shared by apply() and the tensor assembly ------------
 template <typename R, int MODE, int NT>
-static void launch_fwd_x(const DemagGeom& g, const R* m, const R* Ms, const double* Tr, int tsign, cplx_t<R>* X,
-                         int ncomp, const cplx_t<R>* twx, cudaStream_t st) {
-  using C = cplx_t<R>;
-  const int rows = g.ny * g.nz;
-  const int lines = ncomp * rows;
-  if (g.Px == 1) {
-    k_fwd_x1<R, MODE><<<(lines + 255) / 256, 256, 0, st>>>(m, Ms, Tr, X, rows, lines, g.gate);
-    return;
-  }
-  const int nl = x_lines_per_block<R, NT>(lines, g.Lc);
-  const int blocks = (lines + nl - 1) / nl;
-  const int half = nl * (g.Lc | 1);
-  const size_t sm = 2 * sizeof(C) * half;
-  launch_k<FwdX<R, MODE, NT>>(dim3(blocks), sm, st, {m, Ms, Tr, tsign, X, g, lines, nl, twx, half, make_fastdiv(nl), dim3()});
-}
-
-template <typename R, int MODE, int NT>
 static void launch_ypass(const DemagGeom& g, const cplx_t<R>* in, cplx_t<R>* out, const R* Nhat, double* Tq,
                          int ncompc, int ncomp, const cplx_t<R>* twy, int tsign, double tscale, cudaStream_t st) {
   using C = cplx_t<R>;
@@ -933,6 +726,7 @@ static void launch_ypass(const DemagGeom& g, const cplx_t<R>* in, cplx_t<R>* out
   dim3 grid((g.Hx + W - 1) / W, g.nz, ncomp / ncompc);
   const int half = ncompc * W * (g.Py | 1);
   const size_t sm = 2 * sizeof(C) * half;
+  if (sm > 48 * 1024) smem_optin(reinterpret_cast<const void*>(&k_ypass<R, MODE, NT>));
   k_ypass<R, MODE, NT><<<grid, NT, sm, st>>>(in, out, Nhat, Tq, g, ilog2(W), ncompc, twy, tsign, tscale, half);
 }
 
@@ -945,215 +739,40 @@ static void launch_zpass(const DemagGeom& g, cplx_t<R>* Y, const R* Nhat, double
   dim3 grid((g.Hx + W - 1) / W, kyrows, 1);
   const int half = nrow * ncompc * W * (g.Pz | 1);
   const size_t sm = 2 * sizeof(C) * half;
+  if (sm > 48 * 1024) smem_optin(reinterpret_cast<const void*>(&k_zpass<R, MODE, NT>));
   k_zpass<R, MODE, NT><<<grid, NT, sm, st>>>(Y, Nhat, Tq, g, ilog2(W), ncompc, twz, tsign, tscale, half);
-}
-
-// every element offset of the X and Y spectra (3 * nz * max(Py, ny) * Hx
-// complex words) fits in a signed 32-bit int
-static bool offsets_fit_int(const DemagGeom& g) {
-  return 3LL * g.nz * std::max(g.Py, g.ny) * g.Hx < (1LL << 31);
-}
-
-template <typename R>
-static int lines_tile(int Hx, int L, int lines_per_col, int nbuf) {
-  using C = cplx_t<R>;
-  int W = 128 / static_cast<int>(sizeof(C));
-  const size_t per = static_cast<size_t>(std::max(1, nbuf)) * lines_per_col * (L | 1) * sizeof(C);
-  while (W > 1 && W * per > static_cast<size_t>(smem_budget_bytes())) W /= 2;
-  while (W > 1 && W / 2 >= Hx) W /= 2;
-  return W;
-}
-
-// shared memory of one block of a strided pass with tile width W (bytes)
-template <typename R>
-static size_t pass_smem(const DemagGeom& g, int which, bool fused2d, int W) {
-  using C = cplx_t<R>;
-  if (which == 1 || which == 3)
-    return static_cast<size_t>(std::max(1, line_fft_buffers(g.ply))) * sizeof(C) * W *
-           (g.yT ? padded_line_stride(g.Py) : g.Py | 1);
-  if (fused2d) return 2 * sizeof(C) * 3 * W * (g.xT ? padded_line_stride(g.Py) : g.Py | 1);
-  const bool zc2 = (g.Pz & (g.Pz - 1)) == 0 && g.Pz >= 4 && (g.Pz <= 128 || (sizeof(R) == 4 && g.Pz == 256));
-  return (zc2 ? 1 : 2) * sizeof(C) * 3 * W * (g.Pz | 1);
-}
-
-// first radix of the fused-middle z kernel (W * RA threads carry the middle)
-static int zconv2_ra(int Pz) {
-  switch (Pz) {
-    case 4: return 2;
-    case 8: return 4;
-    case 16: return 4;
-    case 32: return 8;
-    case 64: return 8;
-    case 128: return 16;
-    case 256: return 32;
-    default: return 0;
-  }
-}
-
-template <typename R, int MODE>
-static void launch_ylines(const DemagGeom& g, const cplx_t<R>* in, cplx_t<R>* out, const R* Nhat,
-                          const cplx_t<R>* twy, cudaStream_t st, int Wforce = 0) {
-  using C = cplx_t<R>;
-  const int ncompc = MODE == YL_CONV2D ? 3 : 1;
-  const int nbuf = MODE == YL_CONV2D ? 2 : line_fft_buffers(g.ply);
-  const bool xt = MODE == YL_CONV2D ? g.xT != 0 : g.yT != 0;
-  const int W = Wforce > 0 ? Wforce : lines_tile<R>(g.Hx, g.Py, ncompc, nbuf);
-  const int half = ncompc * W * (xt ? padded_line_stride(g.Py) : g.Py | 1);
-  // full tiles; up to W/4 leftover columns (row-major) run as one-column blocks
-  const int rem = g.Hx % W;
-  const int nfull = !xt && rem > 0 && rem <= W / 4 ? g.Hx / W : (g.Hx + W - 1) / W;
-  const int ncols = nfull * W >= g.Hx ? 0 : g.Hx - nfull * W;
-  dim3 grid(nfull + ncols, g.nz, 3 / ncompc);
-  const size_t sm = static_cast<size_t>(std::max(1, nbuf)) * sizeof(C) * half;
-  const FastDiv fnl = make_fastdiv(ncompc * W), fnl1 = make_fastdiv(ncompc);
-  if (xt) {
-    if (offsets_fit_int(g))
-      launch_k<YLines<R, MODE, kHotNT, true, true>>(grid, sm, st, {in, out, Nhat, g, ilog2(W), ncompc, fnl, twy, half, nfull, fnl1, dim3()});
-    else
-      launch_k<YLines<R, MODE, kHotNT, false, true>>(grid, sm, st, {in, out, Nhat, g, ilog2(W), ncompc, fnl, twy, half, nfull, fnl1, dim3()});
-    return;
-  }
-  if (offsets_fit_int(g))
-    launch_k<YLines<R, MODE, kHotNT, true>>(grid, sm, st, {in, out, Nhat, g, ilog2(W), ncompc, fnl, twy, half, nfull, fnl1, dim3()});
-  else
-    launch_k<YLines<R, MODE, kHotNT, false>>(grid, sm, st, {in, out, Nhat, g, ilog2(W), ncompc, fnl, twy, half, nfull, fnl1, dim3()});
-}
-
-template <typename R, int RA, int RB>
-static void launch_zconv2(const DemagGeom& g, cplx_t<R>* Y, const R* Nhat, const cplx_t<R>* twz, cudaStream_t st,
-                          int Wforce) {
-  using C = cplx_t<R>;
-  constexpr int L = RA * RB;
-  constexpr int NTZ = zconv2_nt<R>();
-  // tiles of W columns along kx, or along ky for column-major spectra (yT)
-  int W = Wforce > 0 ? Wforce : lines_tile<R>(g.yT ? g.Py : g.Hx, L, 3, 1);
-  while (W * RA > NTZ) W /= 2;
-  const size_t sm = sizeof(C) * 3 * W * (L | 1);
-  {
-    static std::mutex mu;
-    static uint64_t done = 0;
-    int dev = 0;
-    cudaGetDevice(&dev);
-    const bool tracked = dev >= 0 && dev < 64;
-    std::lock_guard<std::mutex> lk(mu);
-    if (!tracked || !((done >> dev) & 1ull)) {
-      const int mx = static_cast<int>(kMaxSmem);
-      cudaFuncSetAttribute(k_zconv2<R, RA, RB, NTZ, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, mx);
-      cudaFuncSetAttribute(k_zconv2<R, RA, RB, NTZ, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, mx);
-      cudaFuncSetAttribute(k_zconv2<R, RA, RB, NTZ, true, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, mx);
-      cudaFuncSetAttribute(k_zconv2<R, RA, RB, NTZ, false, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, mx);
-      if (tracked) done |= 1ull << dev;
-    }
-  }
-  const FastDiv fnl = make_fastdiv(3 * W);
-  if (g.yT) {
-    dim3 grid(g.Hx, (g.Py + W - 1) / W, 1);
-    if (offsets_fit_int(g))
-      launch_pdl(k_zconv2<R, RA, RB, NTZ, true, true>, grid, dim3(NTZ), sm, st, Y, Nhat, g, ilog2(W), fnl, twz, g.Hx);
-    else
-      launch_pdl(k_zconv2<R, RA, RB, NTZ, false, true>, grid, dim3(NTZ), sm, st, Y, Nhat, g, ilog2(W), fnl, twz, g.Hx);
-    return;
-  }
-  // full kx tiles; up to W/4 leftover columns run as ky tiles in the same grid
-  const int rem = g.Hx % W;
-  const int nfull = rem > 0 && rem <= W / 4 && W <= g.Py ? g.Hx / W : (g.Hx + W - 1) / W;
-  const int ncols = nfull * W >= g.Hx ? 0 : g.Hx - nfull * W;
-  dim3 grid(nfull + ncols, g.Py, 1);
-  if (offsets_fit_int(g))
-    launch_pdl(k_zconv2<R, RA, RB, NTZ, true>, grid, dim3(NTZ), sm, st, Y, Nhat, g, ilog2(W), fnl, twz, nfull);
-  else
-    launch_pdl(k_zconv2<R, RA, RB, NTZ, false>, grid, dim3(NTZ), sm, st, Y, Nhat, g, ilog2(W), fnl, twz, nfull);
-}
-
-// Power-of-two z lengths with a fused-middle kernel: L = RA * RB
-template <typename R>
-static bool try_zconv2(const DemagGeom& g, cplx_t<R>* Y, const R* Nhat, const cplx_t<R>* twz, cudaStream_t st,
-                       int Wf) {
-  switch (g.Pz) {
-    case 4: launch_zconv2<R, 2, 2>(g, Y, Nhat, twz, st, Wf); return true;
-    case 8: launch_zconv2<R, 4, 2>(g, Y, Nhat, twz, st, Wf); return true;
-    case 16: launch_zconv2<R, 4, 4>(g, Y, Nhat, twz, st, Wf); return true;
-    case 32: launch_zconv2<R, 8, 4>(g, Y, Nhat, twz, st, Wf); return true;
-    case 64: launch_zconv2<R, 8, 8>(g, Y, Nhat, twz, st, Wf); return true;
-    case 128: launch_zconv2<R, 16, 8>(g, Y, Nhat, twz, st, Wf); return true;
-    case 256:
-      if constexpr (sizeof(R) == 4) {
-        launch_zconv2<R, 32, 8>(g, Y, Nhat, twz, st, Wf);
-        return true;
-      }
-      return false;
-    default: return false;
-  }
-}
-
-template <typename R, int PZ>
-static void launch_zsmall_pz(const DemagGeom& g, cplx_t<R>* Y, const R* Nhat, cudaStream_t st) {
-  typename ZSmall<R, PZ>::Args a{};
-  a.Y = Y;
-  a.Nhat = Nhat;
-  a.Hx = g.Hx;
-  a.Py = g.Py;
-  a.nz = g.nz;
-  a.Tyq = g.Tyq;
-  a.Tzq = g.Tzq;
-  for (int t = 0; t < PZ; ++t) {
-    const long double ang = -2.0L * 3.141592653589793238462643383279502884L * t / PZ;
-    a.twr[t] = static_cast<R>(static_cast<double>(cosl(ang)));
-    a.twi[t] = static_cast<R>(static_cast<double>(sinl(ang)));
-  }
-  const int64_t lines = static_cast<int64_t>(g.Hx) * g.Py;
-  launch_k<ZSmall<R, PZ>>(dim3(static_cast<unsigned>((lines + 255) / 256)), 0, st, a);
-}
-
-// the direct-DFT z convolution for Pz = 3, 5, 7, 9 on row-major spectra
-template <typename R>
-static bool try_zsmall(const DemagGeom& g, cplx_t<R>* Y, const R* Nhat, cudaStream_t st) {
-  if (g.yT || !zsmall_enabled()) return false;
-  switch (g.Pz) {
-    case 3: launch_zsmall_pz<R, 3>(g, Y, Nhat, st); return true;
-    case 5: launch_zsmall_pz<R, 5>(g, Y, Nhat, st); return true;
-    case 7: launch_zsmall_pz<R, 7>(g, Y, Nhat, st); return true;
-    case 9: launch_zsmall_pz<R, 9>(g, Y, Nhat, st); return true;
-    default: return false;
-  }
-}
-
-template <typename R>
-static void launch_zconv(const DemagGeom& g, cplx_t<R>* Y, const R* Nhat, const cplx_t<R>* twz, cudaStream_t st,
-                         int Wforce, const void* zmap) {
-  using C = cplx_t<R>;
-  if constexpr (sizeof(R) == 4) {
-    if (zpair_enabled() && zpair_applies(g)) {
-      launch_zpair_f32(g, Y, Nhat, zmap, st);
-      return;
-    }
-  } else {
-    if (zquad_applies(g)) {
-      launch_zquad_f64(g, Y, Nhat, st);
-      return;
-    }
-  }
-  if (try_zconv2<R>(g, Y, Nhat, twz, st, Wforce)) return;
-  if (try_zsmall<R>(g, Y, Nhat, st)) return;
-  const int W = Wforce > 0 ? Wforce : lines_tile<R>(g.Hx, g.Pz, 3, 2);
-  const int half = 3 * W * (g.Pz | 1);
-  dim3 grid((g.Hx + W - 1) / W, g.Py, 1);
-  const size_t sm = 2 * sizeof(C) * half;
-  if (offsets_fit_int(g))
-    launch_k<ZConv<R, kHotNT, true>>(grid, sm, st, {Y, Nhat, g, ilog2(W), make_fastdiv(3 * W), twz, half, dim3()});
-  else
-    launch_k<ZConv<R, kHotNT, false>>(grid, sm, st, {Y, Nhat, g, ilog2(W), make_fastdiv(3 * W), twz, half, dim3()});
 }
 
 template <typename R>
 static bool run_pass(const DemagPlan<R>& p, DemagGeom g, int which, const R* m, const R* mu0Ms, R* Hd,
-                     cudaStream_t st) {
+                     cudaStream_t st, bool runtime_len = false) {
   using C = cplx_t<R>;
   constexpr int NT = kHotNT;
   const int64_t xlines = 3LL * g.ny * g.nz, ncz = 3LL * g.nz;
   if (g.wreg && which != 2) {
     launch_wreg(which, g, m, mu0Ms, p.X, p.Y, Hd, p.twx, p.twy, st);
     return true;
+  }
+  if (p.rfft && !runtime_len) {
+    const int rows = g.ny * g.nz;
+    switch (which) {
+      case 0: rf::fwd_x<R>(g.Lc, m, mu0Ms, p.X, p.rtx, p.twx, g.gate, g.nx, rows, g.xT, st); return true;
+      case 1:
+        if (p.fused2d) return false;
+        rf::fwd_y<R>(g.Py, p.X, p.Y, p.rty, g.gate, g.ny, g.nz, g.Hx, st);
+        return true;
+      case 2:
+        if (p.fused2d) rf::conv_film<R>(g.Py, p.X, p.Nhat, p.rty, g.gate, g.ny, g.Hx, st);
+        else if (p.rfft_z) rf::conv_z<R>(g.Pz, p.Y, p.Nhat, p.rtz, g.gate, g.nz, g.Hx, g.Py, st);
+        else launch_zconv<R>(g, p.Y, p.Nhat, p.twz, st, p.tile[2], p.zmap);
+        return true;
+      case 3:
+        if (p.fused2d) return false;
+        rf::inv_y<R>(g.Py, p.Y, p.X, p.rty, g.gate, g.ny, g.nz, g.Hx, st);
+        return true;
+      case 4: rf::inv_x<R>(g.Lc, p.X, Hd, p.rtx, p.twx, g.gate, g.nx, rows, g.xT, st); return true;
+      default: return false;
+    }
   }
   switch (which) {
     case 0:
@@ -1179,7 +798,7 @@ static bool run_pass(const DemagPlan<R>& p, DemagGeom g, int which, const R* m, 
       launch_ylines<R, YL_FWD>(g, p.X, p.Y, p.Nhat, p.twy, st, p.tile[1]);
       return true;
     case 2:
-      if (p.fused2d) launch_ylines<R, YL_CONV2D>(g, p.X, p.X, p.Nhat, p.twy, st, p.tile[2]);
+      if (p.fused2d) launch_ylines<R, YL_CONV2D>(g, p.X, p.X, p.Nhat, p.twy, st, runtime_len ? 0 : p.tile[2]);
       else if (p.long_y && g.Pz == 1)
         k_gproduct_film<R><<<gblocks(static_cast<int64_t>(g.Py) * g.Hx), 256, 0, st>>>(p.Y, p.Nhat, g.Py, g.Hx, g.Tyq,
                                                                                     g.gate);
@@ -1206,10 +825,7 @@ static bool run_pass(const DemagPlan<R>& p, DemagGeom g, int which, const R* m, 
       if (g.Px == 1) {
         k_inv_x1<R><<<(lines + 255) / 256, 256, 0, st>>>(p.X, Hd, lines, g.gate);
       } else {
-        const int nl = x_lines_per_block<R, NT>(lines, g.Lc);
-        const int half = nl * (g.Lc | 1);
-        const size_t sm = 2 * sizeof(C) * half;
-        launch_k<InvX<R, NT>>(dim3((lines + nl - 1) / nl), sm, st, {p.X, Hd, g, lines, nl, p.twx, half, make_fastdiv(nl), dim3()});
+        launch_inv_x<R>(g, p.X, Hd, p.twx, st);
       }
       return true;
     }
@@ -1219,10 +835,10 @@ static bool run_pass(const DemagPlan<R>& p, DemagGeom g, int which, const R* m, 
 }
 
 template <typename R>
-void DemagPlan<R>::apply(const R* m, const R* mu0Ms, R* Hd, cudaStream_t st, const int* gate) {
+void DemagPlan<R>::apply(const R* m, const R* mu0Ms, R* Hd, cudaStream_t st, const int* gate, bool runtime_len) {
   DemagGeom gg = this->g;
   gg.gate = gate;
-  for (int which = 0; which < 5; ++which) run_pass(*this, gg, which, m, mu0Ms, Hd, st);
+  for (int which = 0; which < 5; ++which) run_pass(*this, gg, which, m, mu0Ms, Hd, st, runtime_len && runtime_ok);
 }
 
 template <typename R>
@@ -1267,6 +883,11 @@ int DemagPlan<R>::autotune(const R* m, const R* mu0Ms, R* Hd, cudaStream_t st) {
   const bool zc2 = !fused2d && pass_smem<R>(g, 2, false, 1) == sizeof(C) * 3 * (g.Pz | 1);
   for (int which = 1; which <= 3; ++which) {
     if (fused2d && which != 2) continue;
+    if (rfft && (which != 2 || fused2d || rfft_z)) {  // one width a length
+      const rf::Kind k = which != 2 ? rf::KY : (fused2d ? rf::KC : rf::KZ);
+      tile[which] = rf::tile_width(k, sizeof(R) == 8, which == 2 && !fused2d ? g.Pz : g.Py);
+      continue;
+    }
     if (long_y && (which != 2 || g.Pz == 1)) continue;  // global-memory stages have no tile
     if (g.wreg && which != 2) continue;                  // register passes have no tile
     if (which == 2 && (sizeof(R) == 4 ? zpair_enabled() && zpair_applies(g) : zquad_applies(g))) continue;
@@ -1336,8 +957,8 @@ double DemagPlan<R>::pass_bytes(int which) const {
 template <typename R>
 bool DemagPlan<R>::batchable() const {
   // the paths of run_pass that launch FwdX, YLines, ZConv and InvX only
-  if (long_x || long_y || g.Px == 1 || g.wreg) return false;
-  if (fused2d) return true;
+  if (long_x || (long_y && !rfft) || g.Px == 1 || g.wreg) return false;
+  if (fused2d || rfft_z) return true;
   if (sizeof(R) == 4 && zpair_enabled() && zpair_applies(g)) return false;
   switch (g.Pz) {
     case 4: case 8: case 16: case 32: case 64: case 128: return false;  // k_zconv2

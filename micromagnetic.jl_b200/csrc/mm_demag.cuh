@@ -15,6 +15,7 @@
 // y passes and the product fuse into one y-conv pass.
 #pragma once
 #include "mm_common.cuh"
+#include "mm_rf.cuh"
 
 namespace mm {
 
@@ -58,12 +59,14 @@ class DemagPlan {
   DemagPlan& operator=(const DemagPlan&) = delete;
 
   // Geometry, buffers and twiddle tables.  Returns 0 or a cudaError/-1 (size).
-  int init(int nx, int ny, int nz, cudaStream_t st, char* err, size_t nerr);
+  // runtime_len: the run-time-length passes at their own padded lengths.
+  int init(int nx, int ny, int nz, cudaStream_t st, char* err, size_t nerr, bool runtime_len = false);
   // Tensor spectrum from a real-space FP64 tensor on the device (6 x N,
   // order xx yy zz xy xz yz).
   int set_tensor(const double* T6N_dev, cudaStream_t st);
   // H_demag (SoA 3N) of the magnetisation m (SoA 3N) with mu0*Ms (N).
-  void apply(const R* m, const R* mu0Ms, R* Hd, cudaStream_t st, const int* gate = nullptr);
+  // runtime_len (only where runtime_ok): by the run-time-length passes.
+  void apply(const R* m, const R* mu0Ms, R* Hd, cudaStream_t st, const int* gate = nullptr, bool runtime_len = false);
   // Number of kernel launches of one apply().
   int launches_per_apply() const;
   // Every launch of apply() is a descriptor kernel (mm_launch.cuh), so that a
@@ -86,6 +89,12 @@ class DemagPlan {
 
   DemagGeom g{};
   bool fused2d = false;
+  // x, y and (nz >= 6) z passes on compile-time lengths (mm_rf.cuh), with the
+  // twiddle tables of the x, y (film column) and z lengths
+  bool rfft = false, rfft_z = false;
+  // an rfft film whose buffers and lengths are also those of the run-time passes
+  bool runtime_ok = false;
+  rf::Tw<R> rtx{}, rty{}, rtz{};
   // x / y lines longer than one block holds run as global-memory radix
   // stages (plans gplx / gply, radix <= 8) through ping-pong buffers:
   // S (same shape as Y) for y, Zx / Zx2 ([3 ny nz][Lc]) for x
@@ -101,6 +110,7 @@ class DemagPlan {
   C* twx = nullptr;
   C* twy = nullptr;
   C* twz = nullptr;
+  C* rtab = nullptr;  // storage of rtx, rty, rtz
 
  private:
   size_t bytes_ = 0;
