@@ -374,12 +374,13 @@ __device__ __forceinline__ void llg_rhs(const FieldArgs<R>& a, int64_t I, const 
 // The RK4 / Heun stage update of one cell from its field h at the stage input
 // m: advance_step(::RungeKutta) src/integrator/rk.jl:23-52 and
 // advance_step(::ModifiedEuler) src/integrator/heun.jl:28-49.  mN, mL: the
-// step's start state (hi, lo); av: the accumulator.
-template <typename R>
-__device__ __forceinline__ void rk4_update(const FieldArgs<R>& a, const StageArgs<R>& s, int I, const R m[3],
-                                           const R h[3], const R mN[3], const R mL[3], const R av[3]) {
+// step's start state (hi, lo); av: the accumulator.  out takes what is written:
+// the slope, acc, the next stage input, the state and its low part, component by
+// component.
+template <typename R, class OUT>
+__device__ __forceinline__ void rk4_update_to(const FieldArgs<R>& a, const StageArgs<R>& s, int I, const R m[3],
+                                              const R h[3], const R mN[3], const R mL[3], const R av[3], OUT& out) {
   constexpr bool kF32 = sizeof(R) == 4;
-  const int64_t N = a.N;
   if (s.scheme == 1) {
     // advance_step(::ModifiedEuler)  src/integrator/heun.jl:28-49:
     // k1 = f(m); y = m + h k1; k2 = f(y); m = normalise(m + (h/2) k1 + (h/2) k2)
@@ -389,8 +390,8 @@ __device__ __forceinline__ void rk4_update(const FieldArgs<R>& a, const StageArg
       const R hh = static_cast<R>(s.h);
 #pragma unroll
       for (int c = 0; c < 3; ++c) {
-        s.acc[c * N + I] = f[c];
-        s.ynext[c * N + I] = kF32 ? mN[c] + (mL[c] + hh * f[c]) : mN[c] + hh * f[c];
+        out.acc(c, f[c]);
+        out.ynext(c, kF32 ? mN[c] + (mL[c] + hh * f[c]) : mN[c] + hh * f[c]);
       }
     } else {
       const R h2 = static_cast<R>(0.5 * s.h);
@@ -405,25 +406,27 @@ __device__ __forceinline__ void rk4_update(const FieldArgs<R>& a, const StageArg
         }
         df_normalise(mv, lo);
 #pragma unroll
-        for (int c = 0; c < 3; ++c) s.m_lo[c * N + I] = lo[c];
+        for (int c = 0; c < 3; ++c) out.m_lo(c, lo[c]);
       } else {
 #pragma unroll
         for (int c = 0; c < 3; ++c) mv[c] = mN[c] + h2 * av[c] + h2 * f[c];
         plain_normalise(mv);
       }
 #pragma unroll
-      for (int c = 0; c < 3; ++c) s.m[c * N + I] = mv[c];
+      for (int c = 0; c < 3; ++c) out.m(c, mv[c]);
     }
   } else {
     // advance_step(::RungeKutta)  src/integrator/rk.jl:23-52
     R f[3];
     llg_rhs(a, I, m, h, f);
     const int st = s.stage;
+#pragma unroll
+    for (int c = 0; c < 3; ++c) out.slope(c, f[c]);
     if (st < 4) {
 #pragma unroll
       for (int c = 0; c < 3; ++c) {
         const R kc = f[c];
-        s.acc[c * N + I] = st == 1 ? kc : av[c] + 2 * kc;
+        out.acc(c, st == 1 ? kc : av[c] + 2 * kc);
       }
       const R cf = static_cast<R>(st == 3 ? s.h : 0.5 * s.h);
 #pragma unroll
@@ -431,7 +434,7 @@ __device__ __forceinline__ void rk4_update(const FieldArgs<R>& a, const StageArg
         R v;
         if (kF32) v = mN[c] + (mL[c] + cf * f[c]);
         else v = mN[c] + cf * f[c];
-        s.ynext[c * N + I] = v;
+        out.ynext(c, v);
       }
     } else {
       const R c6 = static_cast<R>(1.0 / 6 * s.h);
@@ -446,16 +449,36 @@ __device__ __forceinline__ void rk4_update(const FieldArgs<R>& a, const StageArg
         }
         df_normalise(mv, lo);
 #pragma unroll
-        for (int c = 0; c < 3; ++c) s.m_lo[c * N + I] = lo[c];
+        for (int c = 0; c < 3; ++c) out.m_lo(c, lo[c]);
       } else {
 #pragma unroll
         for (int c = 0; c < 3; ++c) mv[c] = mN[c] + c6 * (av[c] + f[c]);
         plain_normalise(mv);
       }
 #pragma unroll
-      for (int c = 0; c < 3; ++c) s.m[c * N + I] = mv[c];
+      for (int c = 0; c < 3; ++c) out.m(c, mv[c]);
     }
   }
+}
+
+template <typename R> struct CellOut {  // straight to the arrays
+  const StageArgs<R>& s;
+  int64_t N;
+  int I;
+  // k_i, kept where the adjoint asks for it (k[stage - 1] set)
+  __device__ __forceinline__ void slope(int c, R v) const {
+    if (R* k = s.k[s.stage - 1]) k[c * N + I] = v;
+  }
+  __device__ __forceinline__ void acc(int c, R v) const { s.acc[c * N + I] = v; }
+  __device__ __forceinline__ void ynext(int c, R v) const { s.ynext[c * N + I] = v; }
+  __device__ __forceinline__ void m(int c, R v) const { s.m[c * N + I] = v; }
+  __device__ __forceinline__ void m_lo(int c, R v) const { s.m_lo[c * N + I] = v; }
+};
+template <typename R>
+__device__ __forceinline__ void rk4_update(const FieldArgs<R>& a, const StageArgs<R>& s, int I, const R m[3],
+                                           const R h[3], const R mN[3], const R mL[3], const R av[3]) {
+  CellOut<R> out{s, a.N, I};
+  rk4_update_to(a, s, I, m, h, mN, mL, av, out);
 }
 
 // RK4 / Heun stage, one cell a thread and one z plane a block (k_stage's
@@ -494,14 +517,6 @@ struct StagePlain {
     rk4_update(a, s, I, m, h, mN, mL, av);
   }
 };
-
-// Term sets with a compiled stage kernel of their own (all parameters
-// uniform): exchange + demag (c5), + Zeeman (fig9, c1), exchange + bulk DMI +
-// anisotropy + demag (c2), exchange + interfacial DMI + demag (c3 films)
-constexpr unsigned kFixExDemag = TB_EXCH | TB_DEMAG;
-constexpr unsigned kFixExDemagZee = TB_EXCH | TB_DEMAG | TB_ZEEMAN;
-constexpr unsigned kFixExBulkAnisDemag = TB_EXCH | TB_DMI_BULK | TB_ANIS | TB_DEMAG;
-constexpr unsigned kFixExIntDemag = TB_EXCH | TB_DMI_INTERFACIAL | TB_DEMAG;
 
 template <typename R> struct PersistKind<StagePlain<R>> { static constexpr int value = 11; };
 

@@ -1,9 +1,7 @@
 // mm_field.cu -- fused effective field + LLG + integrator stage kernels.
 #include <cmath>
 
-#include "mm_cell.cuh"
-#include "mm_field.cuh"
-#include "mm_launch.cuh"
+#include "mm_stage.cuh"
 
 namespace mm {
 
@@ -52,233 +50,8 @@ void launch_nbmask(int nx, int ny, int nz, int pbc, const R* Ms, uint8_t* nbm, c
   k_nbmask<R><<<stage_blocks(N), kStageThreads, 0, st>>>(nx, ny, nz, pbc, Ms, nbm);
 }
 
-// Butcher tables of the adaptive methods (src/integrator/adaptive_rk_steps.jl:
-// bs23 11-47, dopri54 49-107, cashkarp54 110-168, fehlberg54 171-229), laid
-// out as RkTableau: rows a[s-1] give the input of stage s+1; row sol-1 is the
-// solution; w are the error weights.
-#define MM_RK_TABLES                                                                                          \
-  {                                                                                                           \
-    {7, 6, 7, 0, 5, 4,                                                                                        \
-     {{1.0 / 5},                                                                                              \
-      {3.0 / 40, 9.0 / 40},                                                                                   \
-      {44.0 / 45, -56.0 / 15, 32.0 / 9},                                                                      \
-      {19372.0 / 6561, -25360.0 / 2187, 64448.0 / 6561, -212.0 / 729},                                        \
-      {9017.0 / 3168, -355.0 / 33, 46732.0 / 5247, 49.0 / 176, -5103.0 / 18656},                              \
-      {35.0 / 384, 0, 500.0 / 1113, 125.0 / 192, -2187.0 / 6784, 11.0 / 84}},                                 \
-     {71.0 / 57600, 0, -71.0 / 16695, 71.0 / 1920, -17253.0 / 339200, 22.0 / 525, -1.0 / 40}},               \
-    {4, 3, 4, 1, 3, 2,                                                                                        \
-     {{0.5}, {0, 0.75}, {2.0 / 9, 1.0 / 3, 4.0 / 9}},                                                         \
-     {-5.0 / 72, 1.0 / 12, 1.0 / 9, -1.0 / 8}},                                                               \
-    {6, 6, 6, 0, 5, 4,                                                                                        \
-     {{1.0 / 5},                                                                                              \
-      {3.0 / 40, 9.0 / 40},                                                                                   \
-      {3.0 / 10, -9.0 / 10, 6.0 / 5},                                                                         \
-      {-11.0 / 54, 5.0 / 2, -70.0 / 27, 35.0 / 27},                                                           \
-      {1631.0 / 55296, 175.0 / 512, 575.0 / 13824, 44275.0 / 110592, 253.0 / 4096},                           \
-      {37.0 / 378, 0, 250.0 / 621, 125.0 / 594, 0, 512.0 / 1771}},                                            \
-     {-277.0 / 64512, 0, 6925.0 / 370944, -6925.0 / 202752, -277.0 / 14336, 277.0 / 7084}},                  \
-    {6, 6, 6, 0, 5, 4,                                                                                        \
-     {{1.0 / 4},                                                                                              \
-      {3.0 / 32, 9.0 / 32},                                                                                   \
-      {1932.0 / 2197, -7200.0 / 2197, 7296.0 / 2197},                                                         \
-      {439.0 / 216, -8.0, 3680.0 / 513, -845.0 / 4104},                                                       \
-      {-8.0 / 27, 2.0, -3544.0 / 2565, 1859.0 / 4104, -11.0 / 40},                                            \
-      {16.0 / 135, 0, 6656.0 / 12825, 28561.0 / 56430, -9.0 / 50, 2.0 / 55}},                                 \
-     {-1.0 / 360, 0, 128.0 / 4275, 2197.0 / 75240, -1.0 / 50, -2.0 / 55}},                                    \
-  }
-
-__constant__ RkTableau c_rk[RK_NMETHODS] = MM_RK_TABLES;
 static const RkTableau h_rk[RK_NMETHODS] = MM_RK_TABLES;
 const RkTableau& rk_tableau(int method) { return h_rk[method]; }
-
-template <typename R, int MODE, bool EXTRA>
-__global__ void __launch_bounds__(kStageThreads, sizeof(R) == 4 ? 3 : 2) k_stage(FieldArgs<R> a, const R* __restrict__ y, StageArgs<R> s) {
-  constexpr bool kF32 = sizeof(R) == 4;
-  pdl_enter();
-  if (MODE == SM_DOPRI && !s.ctrl->active) return;
-  const int64_t N = a.N;
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  const int j = blockIdx.y * blockDim.y + threadIdx.y;
-  const int k = blockIdx.z;
-  const bool live = i < a.nx && j < a.ny;
-  const int I = (k * a.ny + j) * a.nx + i;
-  const int tid = threadIdx.y * blockDim.x + threadIdx.x;
-  const int blin = blockIdx.x + gridDim.x * (blockIdx.y + gridDim.y * blockIdx.z);
-  double e[kNTerms];
-  R m[3], h[3];
-  double red = 0.0;  // SM_DOPRI stage 7: error max
-  // RK4 operands of this cell, loaded together with the field inputs
-  R mN[3], mL[3], av[3];
-  if (MODE == SM_RK4 && live) {
-#pragma unroll
-    for (int c = 0; c < 3; ++c) {
-      mN[c] = s.m[c * N + I];
-      mL[c] = kF32 ? s.m_lo[c * N + I] : R(0);
-      av[c] = s.stage > 1 ? s.acc[c * N + I] : R(0);
-    }
-  }
-  // FSAL: stage 1 takes k1 from the last stage of the accepted attempt
-  const bool reuse = MODE == SM_DOPRI && s.stage == 1 && !s.ctrl->eval1;
-  // SM_DOPRI operands of this cell: the start state, and the earlier slopes
-  // with a non-zero coefficient in this stage's sums.  Loaded together with
-  // the field inputs (walking the tableau row after the field, one dependent
-  // load a term, took 0.270 ms a stage on 256x256x64 FP32 against 0.07 ms of
-  // traffic).
-  R kv[6][3];
-  R co[6];  // a[st-1][j] h (zero: not part of the sum)
-  if constexpr (MODE == SM_DOPRI) {
-    const RkTableau& tb = c_rk[s.method];
-    const int st = s.stage;
-    const double hstep = s.ctrl->step;
-    const bool sum = st <= tb.sol, err = st == tb.err;
-#pragma unroll
-    for (int j = 0; j < 6; ++j) co[j] = static_cast<R>(sum && j < st ? tb.a[st - 1][j] * hstep : 0.0);
-    if (live) {
-#pragma unroll
-      for (int c = 0; c < 3; ++c) {
-        mN[c] = sum ? s.m[c * N + I] : R(0);
-        mL[c] = kF32 && sum ? s.m_lo[c * N + I] : R(0);
-      }
-#pragma unroll
-      for (int j = 0; j < 6; ++j) {
-        const bool need = j < st - 1 && (co[j] != R(0) || (err && tb.w[j] != 0.0));
-#pragma unroll
-        for (int c = 0; c < 3; ++c) kv[j][c] = need ? s.k[j][c * N + I] : R(0);
-      }
-    }
-  }
-  if (live) {
-    if (!reuse) cell_heff<R, MODE == SM_ENERGY || MODE == SM_FIELD, EXTRA>(a, y, I, i, j, k, m, h, e);
-    if (MODE == SM_FIELD) {
-      s.out[I] = h[0];
-      s.out[N + I] = h[1];
-      s.out[2 * N + I] = h[2];
-      if (s.ecell) {
-        double et = 0.0;
-#pragma unroll
-        for (int t = 0; t < kNTerms; ++t) et += e[t];
-        s.ecell[I] = static_cast<R>(et);
-      }
-    } else if (MODE == SM_RHS) {
-      R f[3];
-      llg_rhs(a, I, m, h, f);
-      s.out[I] = f[0];
-      s.out[N + I] = f[1];
-      s.out[2 * N + I] = f[2];
-    } else if (MODE == SM_RK4) {
-      rk4_update(a, s, I, m, h, mN, mL, av);
-    } else if (MODE == SM_DOPRI) {
-      // rk_step_bs23! / rk_step_dopri54! / rk_step_cashkarp54! /
-      // rk_step_fehlberg54!  src/integrator/adaptive_rk_steps.jl:11-229
-      const RkTableau& tb = c_rk[s.method];
-      const int st = s.stage;
-      R f[3];
-      if (reuse) {
-#pragma unroll
-        for (int c = 0; c < 3; ++c) f[c] = s.k[tb.nstage - 1][c * N + I];
-      } else {
-        llg_rhs(a, I, m, h, f);
-      }
-      if (st < tb.err || (tb.fsal && st == tb.nstage)) {
-#pragma unroll
-        for (int c = 0; c < 3; ++c) s.k[st - 1][c * N + I] = f[c];
-      }
-      R yabs[3];  // y_next of the error norm
-      if (st <= tb.sol) {
-        R v[3];
-#pragma unroll
-        for (int c = 0; c < 3; ++c) {
-          R acc = kF32 ? R(0) : mN[c];
-#pragma unroll
-          for (int j = 0; j < 6; ++j) {
-            if (co[j] == R(0)) continue;
-            const R kj = j == st - 1 ? f[c] : kv[j][c];
-            acc = acc + co[j] * kj;
-          }
-          v[c] = acc;
-        }
-        if (st < tb.sol) {
-#pragma unroll
-          for (int c = 0; c < 3; ++c) {
-            if constexpr (kF32) v[c] = mN[c] + (mL[c] + v[c]);
-            s.ynext[c * N + I] = v[c];
-          }
-        } else {
-          // the solution is normalised before it is used (adaptive_rk_steps.jl:35,96,156,217)
-          if constexpr (kF32) {
-            float hi[3], lo[3];
-#pragma unroll
-            for (int c = 0; c < 3; ++c) {
-              hi[c] = mN[c];
-              lo[c] = mL[c];
-              df_add(hi[c], lo[c], v[c]);
-            }
-            df_normalise(hi, lo);
-#pragma unroll
-            for (int c = 0; c < 3; ++c) {
-              s.ynext[c * N + I] = hi[c];
-              s.ynext_lo[c * N + I] = lo[c];
-              yabs[c] = hi[c];
-            }
-          } else {
-            plain_normalise(v);
-#pragma unroll
-            for (int c = 0; c < 3; ++c) {
-              s.ynext[c * N + I] = v[c];
-              yabs[c] = v[c];
-            }
-          }
-        }
-      } else {
-#pragma unroll
-        for (int c = 0; c < 3; ++c) yabs[c] = m[c];
-      }
-      if (st == tb.err) {
-        // error estimate: max |sum_j w_j k_j| / (1 + |y_next|)
-#pragma unroll
-        for (int c = 0; c < 3; ++c) {
-          double et = 0.0;
-#pragma unroll
-          for (int j = 0; j < 7; ++j) {
-            if (j >= st || tb.w[j] == 0.0) continue;
-            const double kj = j == st - 1 || j == 6 ? double(f[c]) : double(kv[j < 6 ? j : 0][c]);
-            et += tb.w[j] * kj;
-          }
-          const double v = fabs(et / (1.0 + fabs(double(yabs[c]))));
-          red = (v > red || isnan(v)) ? v : red;
-        }
-      }
-    }
-  }
-  if (MODE == SM_ENERGY || (MODE == SM_DOPRI && s.stage == c_rk[s.method].err)) {
-    // deterministic block reduction in FP64
-    __shared__ double sh[kStageThreads / 32][kNTerms];
-    const int lane = tid & 31, warp = tid >> 5;
-    constexpr int W = MODE == SM_ENERGY ? kNTerms : 1;
-    double v[W];
-#pragma unroll
-    for (int t = 0; t < W; ++t) v[t] = live ? (MODE == SM_ENERGY ? e[t] : red) : 0.0;
-#pragma unroll
-    for (int t = 0; t < W; ++t) {
-      for (int o = 16; o > 0; o >>= 1) {
-        const double u = __shfl_down_sync(0xffffffffu, v[t], o);
-        if (MODE == SM_ENERGY) v[t] += u;
-        else v[t] = (u > v[t] || isnan(u)) ? u : v[t];
-      }
-      if (lane == 0) sh[warp][t] = v[t];
-    }
-    __syncthreads();
-    if (tid < W) {
-      double acc = 0.0;
-      for (int w = 0; w < kStageThreads / 32; ++w) {
-        const double u = sh[w][tid];
-        if (MODE == SM_ENERGY) acc += u;
-        else acc = (u > acc || isnan(u)) ? u : acc;
-      }
-      s.partials[blin * W + tid] = acc;
-    }
-  }
-}
 
 // RK4 / Heun stage on halo tiles (handles without the further terms): a
 // block of BX x BY threads walks kStageTileZ consecutive z planes of its
@@ -385,11 +158,6 @@ static bool stage_fix_enabled() {
   return on;
 }
 
-template <typename R, unsigned FIX>
-typename StagePlain<R, FIX>::Args fix_args(const typename StagePlain<R>::Args& a) {
-  return {a.a, a.y, a.s, a.bx, a.by, a.grid};
-}
-
 template <typename R>
 bool stage_descriptor_used(const FieldArgs<R>& fa) {
   return !((fa.mask & kExtraBits) || ((fa.mask & TB_DMI_BULK) && fa.x.bD[0]));
@@ -416,23 +184,14 @@ void launch_stage(int mode, const FieldArgs<R>& fa, const R* y, const StageArgs<
                            {fa, y, sa, static_cast<int>(g.block.x), static_cast<int>(g.block.y), dim3()});
     return;
   }
+  // MMCUDA_STAGE_FIX=0 keeps the general kernel
+  const bool uni = !fa.A && !fa.D && !fa.Ku && !fa.Hz && stage_fix_enabled();
   if (mode == SM_RK4) {
-    const typename StagePlain<R>::Args args{fa, y, sa, static_cast<int>(g.block.x), static_cast<int>(g.block.y), dim3()};
-    // a compiled term set when the handle's terms are exactly one of them
-    // with uniform parameters (MMCUDA_STAGE_FIX=0 keeps the general kernel)
-    const bool uni = !fa.A && !fa.D && !fa.Ku && !fa.Hz && stage_fix_enabled();
-    const unsigned fx = uni ? fa.mask : 0u;
-    switch (fx) {
-      case kFixExDemag: launch_k<StagePlain<R, kFixExDemag>>(g.grid, 0, st, fix_args<R, kFixExDemag>(args)); break;
-      case kFixExDemagZee: launch_k<StagePlain<R, kFixExDemagZee>>(g.grid, 0, st, fix_args<R, kFixExDemagZee>(args)); break;
-      case kFixExBulkAnisDemag:
-        launch_k<StagePlain<R, kFixExBulkAnisDemag>>(g.grid, 0, st, fix_args<R, kFixExBulkAnisDemag>(args));
-        break;
-      case kFixExIntDemag: launch_k<StagePlain<R, kFixExIntDemag>>(g.grid, 0, st, fix_args<R, kFixExIntDemag>(args)); break;
-      default: launch_k<StagePlain<R>>(g.grid, 0, st, args); break;
-    }
+    if (uni && launch_rk4_fix<R>(fa, y, sa, g, st)) return;
+    launch_k<StagePlain<R>>(g.grid, 0, st, {fa, y, sa, static_cast<int>(g.block.x), static_cast<int>(g.block.y), dim3()});
     return;
   }
+  if (mode == SM_DOPRI && uni && launch_dopri_fix<R>(fa, y, sa, g, st)) return;
   switch (mode) {
     case SM_FIELD: launch_pdl(k_stage<R, SM_FIELD, false>, g.grid, g.block, 0, st, fa, y, sa); break;
     case SM_RHS: launch_pdl(k_stage<R, SM_RHS, false>, g.grid, g.block, 0, st, fa, y, sa); break;
