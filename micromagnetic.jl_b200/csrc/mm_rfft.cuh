@@ -227,8 +227,9 @@ constexpr Radices radices(int L, int cap = 20) {
       const int m = L / a / b;
       if (!is_radix(m) || m > cap) continue;
       const int mx = a > b ? (a > m ? a : m) : (b > m ? b : m);
-      // largest radix, then the last one, then the even split of the others
-      const int c = mx * 10000 + m * 100 + (a > b ? a - b : b - a);
+      // single lines: the smallest sum of the radices; three components: the
+      // smallest last radix (the most threads a column)
+      const int c = mx * 10000 + (cap == 20 ? (a + b + m) * 100 + m : m * 100 + (a > b ? a - b : b - a));
       if (c < cost) {
         cost = c;
         best = {a, b, m};
@@ -266,8 +267,11 @@ template <typename R_, int L_, int CAP = 20> struct Plan {
 // butterfly tasks t = i * NL + l; else line l at l * LS + a, t = l * NB + i.
 template <class P, int NL, int NT, bool LF> struct Lines {
   using C = typename P::C;
-  static constexpr int LS = P::SIZE + ((P::M - P::SIZE) % P::B + P::B) % P::B;  // line stride (position fastest)
-  static constexpr int kValues = LF ? P::SIZE * NL : LS * NL;               // shared values of a block
+  // interleaved lines fill the banks by themselves: no r padding
+  static constexpr int PB = LF ? P::R3 * P::PA : P::PB;
+  static constexpr int SIZE = LF ? P::R2 * PB : P::SIZE;
+  static constexpr int LS = SIZE + ((P::M - SIZE) % P::B + P::B) % P::B;  // line stride (position fastest)
+  static constexpr int kValues = LF ? SIZE * NL : LS * NL;               // shared values of a block
   static __device__ __forceinline__ int at(int line, int a) { return LF ? a * NL + line : line * LS + a; }
   static constexpr int st = LF ? NL : 1;  // stride of an address step
 
@@ -291,7 +295,7 @@ template <class P, int NL, int NT, bool LF> struct Lines {
       ld(line, i, v);
       dft_half_in<P::R1>(v);
       const int r = i / P::R3, q = i - r * P::R3;
-      C* d = sm + at(line, r * P::PB + q * P::PA);
+      C* d = sm + at(line, r * PB + q * P::PA);
 #pragma unroll
       for (int k = 0; k < P::R1; ++k) d[k * st] = v[k];
     }
@@ -303,7 +307,7 @@ template <class P, int NL, int NT, bool LF> struct Lines {
       int line, i;
       split<P::NB1>(t, line, i);
       const int r = i / P::R3, q = i - r * P::R3;
-      const C* d = sm + at(line, r * P::PB + q * P::PA);
+      const C* d = sm + at(line, r * PB + q * P::PA);
       C v[P::R1];
 #pragma unroll
       for (int k = 0; k < P::R1; ++k) v[k] = d[k * st];
@@ -322,7 +326,7 @@ template <class P, int NL, int NT, bool LF> struct Lines {
         C* d = sm + at(line, q * P::PA + k);
         C v[P::R2];
 #pragma unroll
-        for (int r = 0; r < P::R2; ++r) v[r] = d[r * P::PB * st];
+        for (int r = 0; r < P::R2; ++r) v[r] = d[r * PB * st];
         if (INV) dft<P::R2, true>(v);
 #pragma unroll
         for (int r = 1; r < P::R2; ++r) {
@@ -331,7 +335,7 @@ template <class P, int NL, int NT, bool LF> struct Lines {
         }
         if (!INV) dft<P::R2, false>(v);
 #pragma unroll
-        for (int r = 0; r < P::R2; ++r) d[r * P::PB * st] = v[r];
+        for (int r = 0; r < P::R2; ++r) d[r * PB * st] = v[r];
       }
       __syncthreads();
     }
@@ -339,7 +343,7 @@ template <class P, int NL, int NT, bool LF> struct Lines {
   // the shared values of S3 butterfly i3 of a line: base address, q stride PA
   static __device__ __forceinline__ C* s3_base(C* sm, int line, int i3) {
     const int r = i3 / P::R1, k = i3 - r * P::R1;
-    return sm + at(line, r * P::PB + k);
+    return sm + at(line, r * PB + k);
   }
   static __device__ __forceinline__ void s3(const C* d, int i3, const C* __restrict__ tw3, C* v) {
 #pragma unroll

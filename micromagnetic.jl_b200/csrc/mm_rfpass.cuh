@@ -8,10 +8,11 @@
 // 24 / 19; 300 x 200 x 20: z convolution (40 points) 165 -> 55, y passes 43 ->
 // 23, x passes 50 / 44 -> 28 / 16; 150 x 126 x 37 FP64: z (80 points) 166 -> 68,
 // y 56 -> 22, x 39 / 34 -> 35 / 28; 4000 x 4000 film columns (8000 points) 7 global
-// round trips and a product, 2.7 ms, -> one pass, 0.89 ms.  What bounds them
-// now: instruction issue of the short lines (40 - 60 % active), latency at one
-// block an SM for the 8000-point columns (13 warps), HBM for the y passes of
-// meshes beyond L2 (0.6 of the measured bandwidth).
+// round trips and a product, 2.7 ms, -> one pass, 0.73 ms.  What bounds them
+// now: instruction issue (57 % active in the 2000-point columns, 71 % in the
+// 40-point z convolution), latency at one block an SM for the 8000-point columns
+// (19 warps), HBM and issue together for the y passes of meshes beyond L2 (0.6 of
+// the measured bandwidth).
 //
 // One kernel serves a mesh launched alone and several meshes of a batch in one
 // launch (k_rf): its few arguments are copied to registers, from the
@@ -76,11 +77,26 @@ template <typename C> __device__ __forceinline__ C* dyn_smem() {
   return reinterpret_cast<C*>(rf_smem_raw);
 }
 
-// threads a line of a single-component kernel: one S3 butterfly each while the
-// block stays within `most` threads, else the fewest even rounds that do
-template <class P> constexpr int line_threads(int lines, int most) {
-  const int n = (P::NB3 * lines + most - 1) / most;
-  return (P::NB3 + n - 1) / n;
+// Threads a line of a single-component kernel: the rounds n of S3 butterflies a
+// thread that leave the most warps resident (registers by regs_for; hold: the
+// x passes keep n R3 values across a barrier), fewer rounds where that is within
+// 10 %.  1024 points FP64, 4 lines: 256 threads (2 blocks an SM) 61 / 52 us
+// against 344 threads (1 block) 71 / 65 (1024 x 2048 rows).
+template <class P> constexpr int line_threads(int lines, bool hold, size_t smem) {
+  int best = 0, warps = 0;
+  for (int n = 1; n <= 8; ++n) {
+    const int tl = (P::NB3 + n - 1) / n, nt = (tl * lines + 31) / 32 * 32;
+    const int v = hold && n * P::R3 > P::RMAX ? n * P::R3 : P::RMAX;
+    const int regs = regs_for<typename P::R>(v);
+    if (nt > 1024 || nt * regs > 65536) continue;
+    const int b = blocks_for(nt, regs, smem);
+    const int w = b * nt / 32 - (b == 1 ? 8 : 0);  // a lone block's barriers idle its SM
+    if (best == 0 || 10 * w > 11 * warps) {
+      best = tl;
+      warps = w;
+    }
+  }
+  return best > 0 ? best : (P::NB3 + 7) / 8;
 }
 
 // ------------------------------------------------------------- x passes ---
@@ -97,10 +113,11 @@ template <typename R> constexpr int x_lines(int L) {
 template <typename R, int L> struct XPass {
   using P = Plan<R, L>;
   using C = typename P::C;
-  static constexpr int G = x_lines<R>(L), TL = line_threads<P>(G, sizeof(R) == 4 ? 800 : 400), kNT = G * TL;
+  static constexpr int G = x_lines<R>(L);
+  static constexpr size_t kSmem = sizeof(C) * Lines<P, G, 1, true>::kValues;
+  static constexpr int TL = line_threads<P>(G, true, kSmem), kNT = G * TL;
   static constexpr int NJ3 = (P::NB3 + TL - 1) / TL;
   using S = Lines<P, G, kNT, true>;
-  static constexpr size_t kSmem = sizeof(C) * S::kValues;
   static constexpr int kMinB = blocks_for(kNT, regs_for<R>(P::RMAX > NJ3 * P::R3 ? P::RMAX : NJ3 * P::R3), kSmem);
 };
 
@@ -269,10 +286,11 @@ template <typename R> constexpr int y_cols(int L) {
 template <typename R, int L> struct YPass {
   using P = Plan<R, L>;
   using C = typename P::C;
-  static constexpr int W = y_cols<R>(L), TL = line_threads<P>(W, 512), kNT = W * TL;
+  static constexpr int W = y_cols<R>(L);
+  static constexpr size_t kSmem = sizeof(C) * Lines<P, W, 1, true>::kValues;
+  static constexpr int TL = line_threads<P>(W, false, kSmem), kNT = W * TL;
   static constexpr int NJ3 = (P::NB3 + TL - 1) / TL;
   using S = Lines<P, W, kNT, true>;
-  static constexpr size_t kSmem = sizeof(C) * S::kValues;
   static constexpr int kMinB = blocks_for(kNT, regs_for<R>(P::RMAX), kSmem);
   struct Args {
     const C* in;
@@ -438,14 +456,20 @@ template <typename R> constexpr bool z_has(int L) { return L <= 256 && radices(L
 // Films (nz = 1, column-major X): forward y, tensor product and inverse y of
 // the three components of G columns kx, in place on X.  Position fastest: a
 // column is one contiguous run of memory.
+// SPLIT (columns beyond 4096, one block an SM): the last stage, the product and
+// the first inverse stage as three passes over shared memory instead of 3 R3
+// values in registers, so that the block has 600 threads instead of 400 (the
+// 8000-point columns of a 4000 x 4000 film, where 13 warps issued on 41 % of the
+// cycles: 868 -> 734 us).
 template <typename R, int L> struct FilmConv {
   using P = Plan<R, L, cap3(sizeof(R) == 8, L)>;
   using C = typename P::C;
+  static constexpr bool SPLIT = L > 4096;
   static constexpr int G = P::M >= 96 ? 1 : (96 + P::M - 1) / P::M;
-  static constexpr int kNT = G * P::M;
+  static constexpr int kNT = SPLIT ? 3 * P::M / 2 : G * P::M;
   using S = Lines<P, 3 * G, kNT, false>;
   static constexpr size_t kSmem = sizeof(C) * S::kValues;
-  static constexpr int kMinB = blocks_for(kNT, regs_for<R>(3 * P::R3 > P::RMAX ? 3 * P::R3 : P::RMAX), kSmem);
+  static constexpr int kMinB = blocks_for(kNT, regs_for<R>(!SPLIT && 3 * P::R3 > P::RMAX ? 3 * P::R3 : P::RMAX), kSmem);
   struct Args {
     C* X;
     const R* Nhat;
@@ -467,14 +491,48 @@ template <typename R, int L> struct FilmConv {
     });
     __syncthreads();
     S::template s2<false>(sm, a.tw2);
-    {
+    constexpr int Tyq = L / 2 + 1;
+    const int64_t Ts = static_cast<int64_t>(Hx) * Tyq;
+    if constexpr (SPLIT) {
+      for (int t = threadIdx.x; t < 3 * P::M; t += kNT) {
+        const int c = t / P::M, i3 = t - c * P::M;
+        C* d = S::s3_base(sm, c, i3);
+        C v[P::R3];
+        S::s3(d, i3, a.tw3, v);
+#pragma unroll
+        for (int q = 0; q < P::R3; ++q) d[q * P::PA] = v[q];  // frequency i3 + q M in slot q
+      }
+      __syncthreads();
+      const R* nb = a.Nhat + static_cast<int64_t>(kx0) * Tyq;
+#pragma unroll 4
+      for (int ky = threadIdx.x; ky < L; ky += kNT) {
+        const int q = ky / P::M, i3 = ky - q * P::M;
+        C* d = S::s3_base(sm, 0, i3) + q * P::PA;
+        const bool fy = ky > L / 2;
+        const R sy = fy ? R(-1) : R(1);
+        const R* t = nb + (fy ? L - ky : ky);
+        C x = d[0], y = d[S::LS], z = d[2 * S::LS];
+        tensor_mul<R>(x, y, z, __ldg(t), __ldg(t + Ts), __ldg(t + 2 * Ts), sy * __ldg(t + 3 * Ts), __ldg(t + 4 * Ts),
+                      sy * __ldg(t + 5 * Ts));
+        d[0] = x;
+        d[S::LS] = y;
+        d[2 * S::LS] = z;
+      }
+      __syncthreads();
+      for (int t = threadIdx.x; t < 3 * P::M; t += kNT) {
+        const int c = t / P::M, i3 = t - c * P::M;
+        C* d = S::s3_base(sm, c, i3);
+        C v[P::R3];
+#pragma unroll
+        for (int q = 0; q < P::R3; ++q) v[q] = d[q * P::PA];
+        S::s3_inv(d, i3, a.tw3, v);
+      }
+    } else {
       const int g = threadIdx.x / P::M, i3 = threadIdx.x - g * P::M;
       C v[3][P::R3];
 #pragma unroll
       for (int c = 0; c < 3; ++c) S::s3(S::s3_base(sm, 3 * g + c, i3), i3, a.tw3, v[c]);
       if (kx0 + g < Hx) {
-        constexpr int Tyq = L / 2 + 1;
-        const int64_t Ts = static_cast<int64_t>(Hx) * Tyq;
         const R* nb = a.Nhat + static_cast<int64_t>(kx0 + g) * Tyq;
 #pragma unroll
         for (int q = 0; q < P::R3; ++q) {
