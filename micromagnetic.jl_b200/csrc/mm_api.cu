@@ -131,6 +131,7 @@ class Engine : public EngineBase {
     if (rk_graph) cudaGraphExecDestroy(rk_graph);
     if (dp_graph) cudaGraphExecDestroy(dp_graph);
     if (he_graph) cudaGraphExecDestroy(he_graph);
+    adj_drop_graphs();
     demag.reset();
     demag_sd.reset();
     for (void* p : allocs_) cudaFree(p);
@@ -1224,15 +1225,31 @@ class Engine : public EngineBase {
     int rc;
     const int64_t n3 = 3 * N;
     if (adj_seg_cap < adj_every) {
+      adj_drop_graphs();
       release(adj_seg, adj_seg_cap * n3);
       release(adj_seg_lo, adj_seg_cap * n3);
       adj_seg_cap = 0;
       if ((rc = alloc(adj_seg, adj_every * n3)) || (kF32 && (rc = alloc(adj_seg_lo, adj_every * n3)))) return rc;
       adj_seg_cap = adj_every;
     }
+    // the segment's stage values, where they take at most a quarter of the free
+    // device memory; else the backward walk evaluates the stages again
+    const int64_t steps = std::min(adj_every, adj_n);
+    if (adj_store_cap < steps) {
+      adj_drop_graphs();
+      release(adj_store, adj_store_cap * kAdjVecs * n3);
+      adj_store_cap = 0;
+      size_t fr = 0, tot = 0;
+      MM_CUDA(cudaMemGetInfo(&fr, &tot));
+      if (sizeof(R) * kAdjVecs * n3 * steps <= fr / 4) {
+        if ((rc = alloc(adj_store, steps * kAdjVecs * n3))) return rc;
+        adj_store_cap = steps;
+      }
+    }
+    if (!adj_store && !adj_k[0])
+      for (int i = 0; i < 4; ++i)
+        if ((rc = alloc(adj_Y[i], n3)) || (rc = alloc(adj_k[i], n3)) || (rc = alloc(adj_Hd[i], n3))) return rc;
     if (adj_lam) return MM_OK;
-    for (int i = 0; i < 4; ++i)
-      if ((rc = alloc(adj_Y[i], n3)) || (rc = alloc(adj_k[i], n3)) || (rc = alloc(adj_Hd[i], n3))) return rc;
     if ((rc = alloc(adj_q, n3)) || (rc = alloc(adj_w, n3)) || (rc = alloc(adj_Hdw, n3)) || (rc = alloc(adj_a, n3)) ||
         (rc = alloc(adj_mu, n3)) || (rc = alloc(adj_g, n3)) || (rc = alloc(adj_gMs, N)) || (rc = alloc(adj_gKu, N)) ||
         (rc = alloc(adj_gD, N)) || (rc = alloc(adj_end, n3)) || (kF32 && (rc = alloc(adj_end_lo, n3))) ||
@@ -1263,10 +1280,49 @@ class Engine : public EngineBase {
     }
   }
 
-  // one step backwards: adj_lam holds dL/dy_{n+1} on entry, dL/dy_n on exit
-  void adj_step_back(const R* y, const R* ylo, double h) {
-    adj_recompute_stages(y, ylo, h);
-    const R* const ks[4] = {adj_k[0], adj_k[1], adj_k[2], adj_k[3]};
+  // Stage buffers of one step of a segment: inputs 2..4, slopes and demag
+  // fields of its four stages (11 vectors), kept by adj_forward_step for the
+  // backward walk so that the stages are not evaluated a third time.
+  static constexpr int kAdjVecs = 11;
+  R* adj_slot(int64_t step, int vec) const { return adj_store + (step * kAdjVecs + vec) * 3 * N; }
+
+  // One step of the segment's recomputation with its stage values kept: the
+  // kernels and arithmetic of enqueue_rk4_step.
+  void adj_forward_step(int64_t slot, double h) {
+    FieldArgs<R> fa = fargs(~0u);
+    for (int i = 0; i < 4; ++i) {
+      const R* yin = i == 0 ? m : adj_slot(slot, i - 1);
+      if ((mask & TB_DEMAG) && demag) {
+        fa.Hd = adj_slot(slot, 7 + i);
+        demag->apply(yin, Ms, adj_slot(slot, 7 + i), st_);
+      }
+      StageArgs<R> sa{};
+      sa.m = m;
+      sa.m_lo = m_lo;
+      sa.acc = acc;
+      sa.ynext = i < 3 ? adj_slot(slot, i) : yA;
+      sa.k[i] = adj_slot(slot, 3 + i);
+      sa.h = h;
+      sa.stage = i + 1;
+      launch_stage<R>(SM_RK4, fa, yin, sa, st_);
+    }
+  }
+
+  // one step backwards: adj_lam holds dL/dy_{n+1} on entry, dL/dy_n on exit;
+  // slot >= 0: the step's stage values are kept there
+  void adj_step_back(const R* y, const R* ylo, double h, int64_t slot) {
+    const R* ks[4] = {adj_k[0], adj_k[1], adj_k[2], adj_k[3]};
+    const R* hds[4] = {adj_Hd[0], adj_Hd[1], adj_Hd[2], adj_Hd[3]};
+    if (slot < 0) {
+      adj_recompute_stages(y, ylo, h);
+    } else {
+      adj_Yp[0] = y;
+      for (int i = 0; i < 4; ++i) {
+        if (i > 0) adj_Yp[i] = adj_slot(slot, i - 1);
+        ks[i] = adj_slot(slot, 3 + i);
+        hds[i] = adj_slot(slot, 7 + i);
+      }
+    }
     launch_adj_normalise<R>(y, ylo, ks, h, adj_lam, adj_mu, adj_g, N, st_);
     const unsigned loc = TB_EXCH | TB_DMI_BULK | TB_DMI_INTERFACIAL | TB_ANIS;
     const bool dem = (mask & TB_DEMAG) && demag;
@@ -1275,7 +1331,7 @@ class Engine : public EngineBase {
     static const double wt[4] = {1.0, 2.0, 2.0, 1.0};
     static const double cin[4] = {0.0, 0.5, 0.5, 1.0};
     for (int i = 3; i >= 0; --i) {
-      launch_adj_rhs<R>(fargs(loc), zee, adj_Yp[i], dem ? adj_Hd[i] : nullptr, adj_g, adj_q, adj_w, adj_a, gr, st_);
+      launch_adj_rhs<R>(fargs(loc), zee, adj_Yp[i], dem ? hds[i] : nullptr, adj_g, adj_q, adj_w, adj_a, gr, st_);
       FieldArgs<R> fl = fargs(loc | TB_DEMAG);
       if (dem) {
         demag->apply(adj_w, Ms, adj_Hdw, st_);
@@ -1285,6 +1341,62 @@ class Engine : public EngineBase {
       const double ca = i > 0 ? cin[i] * h : 0.0;
       launch_adj_field<R>(fl, adj_w, adj_q, adj_Yp[i], adj_a, adj_lam, adj_mu, cm, ca, i > 0 ? adj_g : nullptr, gr,
                           st_);
+    }
+  }
+
+  // One segment of len steps from the state in m, forward with its stage values
+  // kept and then backwards: about 55 launches a step.  From the second backward
+  // call on, segments of up to 64 steps replay as a graph.
+  int adj_segment(int64_t len) {
+    auto enqueue = [&]() {
+      const int64_t n3 = 3 * N;
+      for (int64_t s = 0; s < len; ++s) {
+        cudaMemcpyAsync(adj_seg + s * n3, m, sizeof(R) * n3, cudaMemcpyDeviceToDevice, st_);
+        if (kF32) cudaMemcpyAsync(adj_seg_lo + s * n3, m_lo, sizeof(R) * n3, cudaMemcpyDeviceToDevice, st_);
+        adj_forward_step(s, adj_dt);
+      }
+      for (int64_t s = len - 1; s >= 0; --s)
+        adj_step_back(adj_seg + s * n3, kF32 ? adj_seg_lo + s * n3 : nullptr, adj_dt, s);
+    };
+    if (adj_calls == 0 || len > 64) {
+      enqueue();
+      MM_CUDA(cudaGetLastError());
+      return MM_OK;
+    }
+    AdjGraph* g = nullptr;
+    for (AdjGraph& c : adj_graphs)
+      if (c.exec && c.len == len && c.version == version && c.dt == adj_dt) g = &c;
+    if (!g) {
+      // two lengths at most: full segments and the last one
+      g = &adj_graphs[adj_graphs[0].exec && adj_graphs[0].version == version && adj_graphs[0].dt == adj_dt ? 1 : 0];
+      if (g->exec) cudaGraphExecDestroy(g->exec);
+      g->exec = nullptr;
+      cudaGraph_t gr;
+      MM_CUDA(cudaStreamBeginCapture(st_, cudaStreamCaptureModeThreadLocal));
+      enqueue();
+      MM_CUDA(cudaStreamEndCapture(st_, &gr));
+      const cudaError_t e = cudaGraphInstantiate(&g->exec, gr, 0);
+      cudaGraphDestroy(gr);
+      MM_CUDA(e);
+      g->len = len;
+      g->version = version;
+      g->dt = adj_dt;
+    }
+    MM_CUDA(cudaGraphLaunch(g->exec, st_));
+    return MM_OK;
+  }
+  struct AdjGraph {
+    cudaGraphExec_t exec = nullptr;
+    int64_t len = 0;
+    uint64_t version = 0;
+    double dt = 0.0;
+  };
+  AdjGraph adj_graphs[2];
+  int64_t adj_calls = 0;
+  void adj_drop_graphs() {
+    for (AdjGraph& c : adj_graphs) {
+      if (c.exec) cudaGraphExecDestroy(c.exec);
+      c.exec = nullptr;
     }
   }
 
@@ -1312,6 +1424,10 @@ class Engine : public EngineBase {
       const int64_t s0 = sg * adj_every, s1 = std::min(adj_n, s0 + adj_every);
       MM_CUDA(cudaMemcpyAsync(m, adj_ck + sg * n3, sizeof(R) * n3, cudaMemcpyDeviceToDevice, st_));
       if (kF32) MM_CUDA(cudaMemcpyAsync(m_lo, adj_ck_lo + sg * n3, sizeof(R) * n3, cudaMemcpyDeviceToDevice, st_));
+      if (adj_store) {
+        if ((rc = adj_segment(s1 - s0))) return rc;
+        continue;
+      }
       for (int64_t s = s0; s < s1; ++s) {
         MM_CUDA(cudaMemcpyAsync(adj_seg + (s - s0) * n3, m, sizeof(R) * n3, cudaMemcpyDeviceToDevice, st_));
         if (kF32)
@@ -1319,7 +1435,7 @@ class Engine : public EngineBase {
         if (s + 1 < s1 && (rc = rk4_run(adj_dt, 1))) return rc;
       }
       for (int64_t s = s1 - 1; s >= s0; --s)
-        adj_step_back(adj_seg + (s - s0) * n3, kF32 ? adj_seg_lo + (s - s0) * n3 : nullptr, adj_dt);
+        adj_step_back(adj_seg + (s - s0) * n3, kF32 ? adj_seg_lo + (s - s0) * n3 : nullptr, adj_dt, -1);
       MM_CUDA(cudaGetLastError());
     }
     rk_n = rk_n0;
@@ -1336,12 +1452,15 @@ class Engine : public EngineBase {
     if (gKu) MM_CUDA(cudaMemcpyAsync(gKu, adj_gKu, sizeof(double) * N, cudaMemcpyDeviceToHost, st_));
     if (gD) MM_CUDA(cudaMemcpyAsync(gD, adj_gD, sizeof(double) * N, cudaMemcpyDeviceToHost, st_));
     MM_CUDA(cudaStreamSynchronize(st_));
+    ++adj_calls;
     if (hflag) return fail(MM_ERR_NAN, "NaN in dL/dm");
     return MM_OK;
   }
 
   R *adj_ck = nullptr, *adj_ck_lo = nullptr, *adj_seg = nullptr, *adj_seg_lo = nullptr;
   R *adj_Y[4] = {}, *adj_k[4] = {}, *adj_Hd[4] = {};
+  R* adj_store = nullptr;
+  int64_t adj_store_cap = 0;
   const R* adj_Yp[4] = {};
   R *adj_q = nullptr, *adj_w = nullptr, *adj_Hdw = nullptr, *adj_end = nullptr, *adj_end_lo = nullptr;
   double *adj_lam = nullptr, *adj_mu = nullptr, *adj_g = nullptr, *adj_a = nullptr;
