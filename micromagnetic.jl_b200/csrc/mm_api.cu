@@ -1129,33 +1129,35 @@ class Engine : public EngineBase {
       if (!gk && (rc = alloc(gk, 3 * N))) return rc;
       if (!sd && (rc = alloc(sd, 1))) return rc;
       if (kF32) MM_CUDA(cudaMemsetAsync(m_lo, 0, sizeof(R) * 3 * N, st_));
-      SdState hs{0.0, 1.0, 1e-10, sd_steps};
+      SdState hs{0.0, 1.0, 1e-10, sd_steps, 0.0, stop * dmdt_factor, 0, 1};
       MM_CUDA(cudaMemcpyAsync(sd, &hs, sizeof(hs), cudaMemcpyHostToDevice, st_));
       const int nb = stage_blocks(N);
       const bool dm = (mask & TB_DEMAG) && demag;
       DemagPlan<R>* const plan = dm ? sd_plan() : nullptr;
       if (dm && !plan) return MM_ERR_CUDA;
-      for (; i <= max_steps; ++i) {
-        enqueue_thermal(th_step, nullptr, th_dt, nullptr);
-        if (plan) plan->apply(m, Ms, Hd, st_, nullptr, plan->runtime_ok && !kF32);
-        StageArgs<R> sf{};
-        sf.out = work;
-        launch_stage<R>(SM_FIELD, fargs(~0u), m, sf, st_);
-        launch_sd_gk<R>(m, pre, work, gk, N, sd_steps == 0 ? 1 : 0, partials, st_);
-        launch_sd_tau(sd, partials, nb, st_);
-        launch_sd_update<R>(m, pre, work, gk, pins_on ? pins : nullptr, sd, N, st_);
-        launch_sd_count(sd, st_);
-        ++sd_steps;
-        if (sd_steps % 10 == 0) launch_normalise<R>(m, N, st_);
-        launch_max_dm<R>(m, nullptr, pre, nullptr, N, partials + 3 * nb, scal, st_);
-        double out[2];
-        MM_CUDA(cudaMemcpyAsync(&out[0], scal, sizeof(double), cudaMemcpyDeviceToHost, st_));
-        MM_CUDA(cudaMemcpyAsync(&out[1], &sd->tau, sizeof(double), cudaMemcpyDeviceToHost, st_));
+      // iterations are enqueued up to eight at a time; past the stopping one their
+      // kernels return at once
+      int64_t queued = 0;
+      while (hs.active && queued < max_steps) {
+        for (int q = 0; q < 8 && queued < max_steps; ++q, ++queued) {
+          enqueue_thermal(th_step, nullptr, th_dt, nullptr);
+          if (plan) plan->apply(m, Ms, Hd, st_, &sd->active, plan->runtime_ok && !kF32);
+          StageArgs<R> sf{};
+          sf.out = work;
+          launch_stage<R>(SM_FIELD, fargs(~0u), m, sf, st_);
+          launch_sd_gk<R>(m, pre, work, gk, N, sd_steps == 0 ? 1 : 0, partials, sd, st_);
+          launch_sd_tau(sd, partials, nb, st_);
+          launch_sd_update<R>(m, pre, work, gk, pins_on ? pins : nullptr, sd, N, st_);
+          ++sd_steps;
+          if (sd_steps % 10 == 0) launch_sd_normalise<R>(m, N, sd, st_);
+          launch_sd_finish<R>(m, pre, N, partials + 3 * nb, sd, time_factor, st_);
+        }
+        MM_CUDA(cudaMemcpyAsync(&hs, sd, sizeof(hs), cudaMemcpyDeviceToHost, st_));
         MM_CUDA(cudaStreamSynchronize(st_));
-        const double step_size = out[1] / time_factor;
-        max_dmdt = out[0] / step_size;
-        if (max_dmdt < stop * dmdt_factor) break;
+        sd_steps = hs.steps;
       }
+      max_dmdt = hs.max_dmdt;
+      i = hs.active ? max_steps + 1 : hs.iters;
     } else {
       if ((rc = dopri_alloc())) return rc;
       for (; i <= max_steps; ++i) {

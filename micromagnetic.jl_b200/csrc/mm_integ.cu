@@ -106,8 +106,10 @@ void launch_dopri_accept(const DopriCtrl* c, R* m, R* m_lo, const R* yn, const R
 // compute_tau (56-82), run_step_kernel! (39-54).  Sums are FP64.
 template <typename R>
 __global__ void k_sd_gk(const R* __restrict__ m, const R* __restrict__ pre, const R* __restrict__ h,
-                        R* __restrict__ gk, int64_t N, int first, double* __restrict__ partials) {
+                        R* __restrict__ gk, int64_t N, int first, double* __restrict__ partials,
+                        const SdState* __restrict__ s) {
   __shared__ double sh[3][256];
+  if (!s->active) return;
   const int64_t I = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x;
   double ss = 0, sf = 0, ff = 0;
   if (I < N) {
@@ -142,6 +144,7 @@ __global__ void k_sd_gk(const R* __restrict__ m, const R* __restrict__ pre, cons
 // tau from the Barzilai-Borwein sums (compute_tau, src/sd.jl:56-82)
 __global__ void k_sd_tau(SdState* __restrict__ s, const double* __restrict__ partials, int nblocks) {
   __shared__ double sh[3][256];
+  if (!s->active) return;
   if (s->steps == 0) {
     if (threadIdx.x == 0) s->tau = s->min_tau;
     return;
@@ -171,7 +174,7 @@ __global__ void k_sd_update(R* __restrict__ m, R* __restrict__ pre, const R* __r
                             const R* __restrict__ gk, const uint8_t* __restrict__ pins, const SdState* __restrict__ s,
                             int64_t N) {
   const int64_t I = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x;
-  if (I >= N) return;
+  if (I >= N || !s->active) return;
   const R mx = m[I], my = m[N + I], mz = m[2 * N + I];
   pre[I] = mx;
   pre[N + I] = my;
@@ -189,12 +192,10 @@ __global__ void k_sd_update(R* __restrict__ m, R* __restrict__ pre, const R* __r
   m[2 * N + I] = nz / (1 + factor);
 }
 
-__global__ void k_sd_count(SdState* __restrict__ s) { s->steps += 1; }
-
 template <typename R>
-__global__ void k_normalise(R* __restrict__ m, int64_t N) {
+__global__ void k_normalise(R* __restrict__ m, int64_t N, const SdState* __restrict__ s) {
   const int64_t I = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x;
-  if (I >= N) return;
+  if (I >= N || !s->active) return;
   const R x = m[I], y = m[N + I], z = m[2 * N + I];
   const R m2 = x * x + y * y + z * z;
   if (m2 > 0) {
@@ -208,8 +209,10 @@ __global__ void k_normalise(R* __restrict__ m, int64_t N) {
 // max over cells of |a - b| (compute_dm! + maximum, src/helper.jl:273-286)
 template <typename R>
 __global__ void k_max_dm(const R* __restrict__ a, const R* __restrict__ alo, const R* __restrict__ b,
-                         const R* __restrict__ blo, int64_t N, double* __restrict__ partials) {
+                         const R* __restrict__ blo, int64_t N, double* __restrict__ partials,
+                         const int* __restrict__ gate) {
   __shared__ double sh[256];
+  if (gate && !*gate) return;
   const int64_t I = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x;
   double v = 0.0;
   if (I < N) {
@@ -244,6 +247,27 @@ __global__ void k_reduce_max(const double* __restrict__ partials, int nblocks, d
   if (threadIdx.x == 0) *out = sh[0];
 }
 
+// one block: the maximum of the partials and the end of a descent iteration
+__global__ void k_sd_finish(const double* __restrict__ partials, int nblocks, SdState* __restrict__ s,
+                            double time_factor) {
+  __shared__ double sh[256];
+  if (!s->active) return;
+  double v = 0.0;
+  for (int b = threadIdx.x; b < nblocks; b += blockDim.x) v = fmax(v, partials[b]);
+  sh[threadIdx.x] = v;
+  __syncthreads();
+  for (int o = blockDim.x / 2; o > 0; o >>= 1) {
+    if (threadIdx.x < o) sh[threadIdx.x] = fmax(sh[threadIdx.x], sh[threadIdx.x + o]);
+    __syncthreads();
+  }
+  if (threadIdx.x != 0) return;
+  s->steps += 1;
+  s->iters += 1;
+  const double step_size = s->tau / time_factor;
+  s->max_dmdt = sh[0] / step_size;
+  if (s->max_dmdt < s->stop) s->active = 0;
+}
+
 // max_i |v_i| over a 3N vector (compute_initial_step, adaptive_rk.jl:156)
 template <typename R>
 __global__ void k_absmax(const R* __restrict__ v, int64_t n, double* __restrict__ partials) {
@@ -267,8 +291,9 @@ __global__ void k_absmax(const R* __restrict__ v, int64_t n, double* __restrict_
 }
 
 template <typename R>
-void launch_sd_gk(const R* m, const R* pre, const R* h, R* gk, int64_t N, int first, double* partials, cudaStream_t st) {
-  k_sd_gk<R><<<stage_blocks(N), 256, 0, st>>>(m, pre, h, gk, N, first, partials);
+void launch_sd_gk(const R* m, const R* pre, const R* h, R* gk, int64_t N, int first, double* partials, const SdState* s,
+                  cudaStream_t st) {
+  k_sd_gk<R><<<stage_blocks(N), 256, 0, st>>>(m, pre, h, gk, N, first, partials, s);
 }
 void launch_sd_tau(SdState* s, const double* partials, int nblocks, cudaStream_t st) {
   k_sd_tau<<<1, 256, 0, st>>>(s, partials, nblocks);
@@ -277,15 +302,21 @@ template <typename R>
 void launch_sd_update(R* m, R* pre, const R* h, const R* gk, const uint8_t* pins, const SdState* s, int64_t N, cudaStream_t st) {
   k_sd_update<R><<<stage_blocks(N), 256, 0, st>>>(m, pre, h, gk, pins, s, N);
 }
-void launch_sd_count(SdState* s, cudaStream_t st) { k_sd_count<<<1, 1, 0, st>>>(s); }
 template <typename R>
-void launch_normalise(R* m, int64_t N, cudaStream_t st) {
-  k_normalise<R><<<stage_blocks(N), 256, 0, st>>>(m, N);
+void launch_sd_normalise(R* m, int64_t N, const SdState* s, cudaStream_t st) {
+  k_normalise<R><<<stage_blocks(N), 256, 0, st>>>(m, N, s);
+}
+template <typename R>
+void launch_sd_finish(const R* m, const R* pre, int64_t N, double* partials, SdState* s, double time_factor,
+                      cudaStream_t st) {
+  const int nb = stage_blocks(N);
+  k_max_dm<R><<<nb, 256, 0, st>>>(m, nullptr, pre, nullptr, N, partials, &s->active);
+  k_sd_finish<<<1, 256, 0, st>>>(partials, nb, s, time_factor);
 }
 template <typename R>
 void launch_max_dm(const R* a, const R* alo, const R* b, const R* blo, int64_t N, double* partials, double* out, cudaStream_t st) {
   const int nb = stage_blocks(N);
-  k_max_dm<R><<<nb, 256, 0, st>>>(a, alo, b, blo, N, partials);
+  k_max_dm<R><<<nb, 256, 0, st>>>(a, alo, b, blo, N, partials, nullptr);
   k_reduce_max<<<1, 256, 0, st>>>(partials, nb, out);
 }
 template <typename R>
@@ -296,10 +327,12 @@ void launch_absmax(const R* v, int64_t n, double* partials, double* out, cudaStr
 
 #define MM_INST2(R)                                                                                          \
   template void launch_dopri_accept<R>(const DopriCtrl*, R*, R*, const R*, const R*, int64_t, cudaStream_t); \
-  template void launch_sd_gk<R>(const R*, const R*, const R*, R*, int64_t, int, double*, cudaStream_t);      \
+  template void launch_sd_gk<R>(const R*, const R*, const R*, R*, int64_t, int, double*, const SdState*,     \
+                                cudaStream_t);                                                               \
   template void launch_sd_update<R>(R*, R*, const R*, const R*, const uint8_t*, const SdState*, int64_t,     \
                                     cudaStream_t);                                                           \
-  template void launch_normalise<R>(R*, int64_t, cudaStream_t);                                              \
+  template void launch_sd_normalise<R>(R*, int64_t, const SdState*, cudaStream_t);                           \
+  template void launch_sd_finish<R>(const R*, const R*, int64_t, double*, SdState*, double, cudaStream_t);   \
   template void launch_max_dm<R>(const R*, const R*, const R*, const R*, int64_t, double*, double*,          \
                                  cudaStream_t);                                                              \
   template void launch_absmax<R>(const R*, int64_t, double*, double*, cudaStream_t);
