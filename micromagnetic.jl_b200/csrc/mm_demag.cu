@@ -264,18 +264,23 @@ void smem_optin(const void* kernel) {
   done.insert({kernel, dev});
 }
 
+// exp(-2 pi i t / L), t < L; Q > 0 (L = 64 Q, the register passes): followed by
+// their table exp(-2 pi i q k / (L / 2)) at k Q + q, k < 32, q < Q
 template <typename C>
-static C* upload_twiddles(int L, size_t& bytes, cudaStream_t st) {
+static C* upload_twiddles(int L, size_t& bytes, cudaStream_t st, int Q = 0) {
   std::vector<C> h(L);
   for (int t = 0; t < L; ++t) {
     const long double a = -2.0L * 3.141592653589793238462643383279502884L * t / L;
     h[t].x = static_cast<decltype(C::x)>(static_cast<double>(cosl(a)));
     h[t].y = static_cast<decltype(C::x)>(static_cast<double>(sinl(a)));
   }
+  for (int k = 0; k < (Q > 0 ? 32 : 0); ++k)
+    for (int q = 0; q < Q; ++q) h.push_back(h[2 * q * k]);
+  const int n = static_cast<int>(h.size());
   C* d = nullptr;
-  if (cudaMalloc(&d, sizeof(C) * L) != cudaSuccess) return nullptr;
-  bytes += sizeof(C) * L;
-  cudaMemcpyAsync(d, h.data(), sizeof(C) * L, cudaMemcpyHostToDevice, st);
+  if (cudaMalloc(&d, sizeof(C) * n) != cudaSuccess) return nullptr;
+  bytes += sizeof(C) * n;
+  cudaMemcpyAsync(d, h.data(), sizeof(C) * n, cudaMemcpyHostToDevice, st);
   cudaStreamSynchronize(st);
   return d;
 }
@@ -448,8 +453,8 @@ int DemagPlan<R>::init(int nx, int ny, int nz, cudaStream_t st, char* err, size_
       return -1;
     }
   }
-  if (g.Px > 1 && !(twx = upload_twiddles<C>(g.Px, bytes_, st))) return 2;
-  if (!(twy = upload_twiddles<C>(g.Py, bytes_, st))) return 2;
+  if (g.Px > 1 && !(twx = upload_twiddles<C>(g.Px, bytes_, st, g.wreg ? nx / 32 : 0))) return 2;
+  if (!(twy = upload_twiddles<C>(g.Py, bytes_, st, g.wreg ? ny / 32 : 0))) return 2;
   if (!(twz = upload_twiddles<C>(g.Pz, bytes_, st))) return 2;
   if (rfft) {
     std::vector<C> h;

@@ -96,7 +96,7 @@ __global__ void __launch_bounds__(32 * W, (x_fwd_minb<R, W>())) k_xfwd_w(const R
       }
     }
     if (c > 0) __syncthreads();  // the previous component's staged rows are written out
-    wfft<Q, false, 2>(v, sm + warp * wtile_size<Q>(), twx);
+    wfft<Q, false>(v, sm + warp * wtile_size<Q>(), twx + 64 * Q);
     __syncthreads();  // every warp is done with its transpose tile
 #pragma unroll
     for (int r = 0; r < 32; ++r) sm[(q + Q * (r / Q) + 32 * (r % Q)) * S + rl] = v[r];
@@ -169,7 +169,7 @@ __global__ void __launch_bounds__(32 * W, (x_inv_minb<R, W>())) k_xinv_w(const c
     v[j] = cmk<C>(a.x + b.x - d.y, a.y + b.y + d.x);
   }
   __syncthreads();  // the staging tile becomes the transpose tiles
-  wfft<Q, true, 2>(v, sm + warp * wtile_size<Q>(), twx);
+  wfft<Q, true>(v, sm + warp * wtile_size<Q>(), twx + 64 * Q);
   // z[n] = (x[2n], x[2n+1]) for n < Lc / 2: registers with k2 = r % Q < Q / 2
   C* h2 = reinterpret_cast<C*>(H + c * N + static_cast<int64_t>(row0 + rl) * nx);
 #pragma unroll
@@ -202,7 +202,7 @@ __global__ void __launch_bounds__(kWyNT, 3) k_yfwd_w(const float2* __restrict__ 
     if (s) a = cmul(a, __ldg(twy + q + Q * j));
     v[j] = a;
   }
-  wfft<Q, false, 2>(v, smy + warp * wtile_size<Q>(), twy);
+  wfft<Q, false>(v, smy + warp * wtile_size<Q>(), twy + 64 * Q);
   __syncthreads();  // transposes done: the tiles become the block's output columns
   // Y[2k + s] of line ll staged as half column (ll, s), k contiguous
   float2* half = smy + (2 * ll + s) * (Py / 2);
@@ -248,7 +248,7 @@ __global__ void __launch_bounds__(kWyNT, 3) k_yinv_w(const float2* __restrict__ 
 #pragma unroll
   for (int j = 0; j < 32; ++j) v[j] = ll < nl ? col[q + Q * j] : make_float2(0.f, 0.f);
   __syncthreads();  // the staged columns become the transpose tiles
-  wfft<Q, true, 2>(v, smy + warp * wtile_size<Q>(), twy);
+  wfft<Q, true>(v, smy + warp * wtile_size<Q>(), twy + 64 * Q);
   if (s) {
 #pragma unroll
     for (int r = 0; r < 32; ++r) {
@@ -309,7 +309,7 @@ __global__ void __launch_bounds__(kWdNT, 3) k_yfwd_d(const float2* __restrict__ 
     if (s) a = cmul(a, __ldg(twy + q + Q * j));
     v[j] = a;
   }
-  wfft<Q, false, 2>(v, tiles + warp * wtile_size<Q>(), twy);
+  wfft<Q, false>(v, tiles + warp * wtile_size<Q>(), twy + 64 * Q);
   float2* yc = Y + static_cast<int64_t>(line) * Py + s;
 #pragma unroll
   for (int r = 0; r < 32; ++r) yc[2 * (q + Q * (r / Q) + 32 * (r % Q))] = v[r];
@@ -334,7 +334,7 @@ __global__ void __launch_bounds__(kWdNT, 3) k_yinv_d(const float2* __restrict__ 
 #pragma unroll
   for (int j = 0; j < 32; ++j) v[j] = yc[2 * (q + Q * j)];
   float2* tile = tiles + warp * wtile_size<Q>();
-  wfft<Q, true, 2>(v, tile, twy);
+  wfft<Q, true>(v, tile, twy + 64 * Q);
   if (s) {
 #pragma unroll
     for (int r = 0; r < 32; ++r) {
@@ -474,7 +474,7 @@ __global__ void __launch_bounds__(kWpNT, sizeof(R) == 4 ? 8 : 4) k_yfwd_p(const 
     __syncthreads();  // both warps hold the line: the buffer takes the next one
     if (threadIdx.x == 0 && line + static_cast<int>(gridDim.x) < nlines)
       bulk_load(buf, X + static_cast<int64_t>(line + gridDim.x) * NY, NY * sizeof(C), bar);
-    wfft<32, false, 2>(v, tile, twy);
+    wfft<32, false>(v, tile, twy + 64 * 32);
     // the two parities interleave in the tiles' space (2048 values), which
     // leave as one copy (Y[2k], Y[2k + 1], ...)
     __syncthreads();
@@ -530,7 +530,7 @@ __global__ void __launch_bounds__(kWpNT, sizeof(R) == 4 ? 6 : 3) k_yinv_p(const 
     __syncthreads();  // both warps hold the line (and are done with last line's tiles)
     if (threadIdx.x == 0 && line + static_cast<int>(gridDim.x) < nlines)
       bulk_load(buf, Y + static_cast<int64_t>(line + gridDim.x) * Py, Py * sizeof(C), bar);
-    wfft<32, true, 2>(v, tile, twy);
+    wfft<32, true>(v, tile, twy + 64 * 32);
     if (s) {
 #pragma unroll
       for (int r = 0; r < 32; ++r) {
