@@ -280,10 +280,10 @@ int mm_rk4_launches_per_step(mm_handle* h, int* launches);
 /* ---- batches: several meshes (ensembles, NEB images) stepped together ----
  * The reference evaluates NEB images one after another (src/neb/neb.jl:220-232).
  * A batch captures one RK4 step of every handle (same device, same dt) in one
- * CUDA graph and replays it once per step: the demag passes and stage
- * kernels of meshes that take the shared-memory FFT paths are launched once
- * per pass for all of them (mm_batch_launches), other meshes run as parallel
- * branches of the graph; work
+ * CUDA graph and replays it once per step: meshes with the same kernels (small
+ * meshes of any sizes; larger ones of equal line lengths) share one launch per
+ * pass (mm_batch_launches), the others run as parallel branches of the graph;
+ * work
  * queued on the handles before mm_batch_rk4_run precedes the batch and work
  * queued after it follows.  The handles stay owned by the caller and must
  * outlive the batch. */
