@@ -1203,6 +1203,11 @@ class Engine : public EngineBase {
     adj_every = ck;
     adj_nck = nck;
     adj_dt = dt;
+    if (const AdjKey key{n, ck, version, dt}; !(key == adj_key)) {
+      adj_drop_graphs();
+      adj_key = key;
+      adj_calls = 0;
+    }
     for (int64_t s = 0; s < n; ++s) {
       if (s % ck == 0) {
         const int64_t slot = s / ck;
@@ -1347,8 +1352,11 @@ class Engine : public EngineBase {
   }
 
   // One segment of len steps from the state in m, forward with its stage values
-  // kept and then backwards: about 55 launches a step.  From the second backward
-  // call on, segments of up to 64 steps replay as a graph.
+  // kept and then backwards: about 55 launches a step.  Segments of up to 64
+  // steps replay as a graph where an earlier backward call had the same steps,
+  // spacing, time step and parameters: a loop that changes a parameter, the
+  // number of steps or the spacing before every record would capture and
+  // instantiate thousands of nodes for one use, so it launches directly.
   int adj_segment(int64_t len) {
     auto enqueue = [&]() {
       const int64_t n3 = 3 * N;
@@ -1365,40 +1373,35 @@ class Engine : public EngineBase {
       MM_CUDA(cudaGetLastError());
       return MM_OK;
     }
-    AdjGraph* g = nullptr;
-    for (AdjGraph& c : adj_graphs)
-      if (c.exec && c.len == len && c.version == version && c.dt == adj_dt) g = &c;
-    if (!g) {
-      // two lengths at most: full segments and the last one
-      g = &adj_graphs[adj_graphs[0].exec && adj_graphs[0].version == version && adj_graphs[0].dt == adj_dt ? 1 : 0];
-      if (g->exec) cudaGraphExecDestroy(g->exec);
-      g->exec = nullptr;
+    cudaGraphExec_t& exec = adj_graphs[len == adj_every ? 0 : 1];  // full segments, the last one
+    if (!exec) {
       cudaGraph_t gr;
       MM_CUDA(cudaStreamBeginCapture(st_, cudaStreamCaptureModeThreadLocal));
       enqueue();
       MM_CUDA(cudaStreamEndCapture(st_, &gr));
-      const cudaError_t e = cudaGraphInstantiate(&g->exec, gr, 0);
+      const cudaError_t e = cudaGraphInstantiate(&exec, gr, 0);
       cudaGraphDestroy(gr);
+      if (e != cudaSuccess) exec = nullptr;
       MM_CUDA(e);
-      g->len = len;
-      g->version = version;
-      g->dt = adj_dt;
     }
-    MM_CUDA(cudaGraphLaunch(g->exec, st_));
+    MM_CUDA(cudaGraphLaunch(exec, st_));
     return MM_OK;
   }
-  struct AdjGraph {
-    cudaGraphExec_t exec = nullptr;
-    int64_t len = 0;
+  // what the segment graphs were captured for
+  struct AdjKey {
+    int64_t n = 0, every = 0;
     uint64_t version = 0;
     double dt = 0.0;
+    bool operator==(const AdjKey&) const = default;
   };
-  AdjGraph adj_graphs[2];
-  int64_t adj_calls = 0;
+  AdjKey adj_key;
+  cudaGraphExec_t adj_graphs[2] = {};
+  int64_t adj_calls = 0;  // backward calls finished with adj_key
+  // (after the stream has drained)
   void adj_drop_graphs() {
-    for (AdjGraph& c : adj_graphs) {
-      if (c.exec) cudaGraphExecDestroy(c.exec);
-      c.exec = nullptr;
+    for (cudaGraphExec_t& e : adj_graphs) {
+      if (e) cudaGraphExecDestroy(e);
+      e = nullptr;
     }
   }
 
