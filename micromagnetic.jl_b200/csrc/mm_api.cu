@@ -65,6 +65,15 @@ __global__ void k_to_double(const R* __restrict__ a, double* __restrict__ b, int
   if (i < n) b[i] = static_cast<double>(a[i]);
 }
 
+// MMCUDA_ADJ_STORE=0: gradients keep no stage values
+static bool adj_store_enabled() {
+  static const bool on = [] {
+    const char* e = getenv("MMCUDA_ADJ_STORE");
+    return !(e && e[0] == '0');
+  }();
+  return on;
+}
+
 class EngineBase {
  public:
   virtual ~EngineBase() = default;
@@ -1240,7 +1249,8 @@ class Engine : public EngineBase {
       adj_seg_cap = adj_every;
     }
     // the segment's stage values, where they take at most a quarter of the free
-    // device memory; else the backward walk evaluates the stages again
+    // device memory; else, or when the allocation fails, the backward walk
+    // evaluates the stages again
     const int64_t steps = std::min(adj_every, adj_n);
     if (adj_store_cap < steps) {
       adj_drop_graphs();
@@ -1248,9 +1258,9 @@ class Engine : public EngineBase {
       adj_store_cap = 0;
       size_t fr = 0, tot = 0;
       MM_CUDA(cudaMemGetInfo(&fr, &tot));
-      if (sizeof(R) * kAdjVecs * n3 * steps <= fr / 4) {
-        if ((rc = alloc(adj_store, steps * kAdjVecs * n3))) return rc;
-        adj_store_cap = steps;
+      if (adj_store_enabled() && sizeof(R) * kAdjVecs * n3 * steps <= fr / 4) {
+        if (alloc(adj_store, steps * kAdjVecs * n3) == MM_OK) adj_store_cap = steps;
+        else cudaGetLastError();
       }
     }
     if (!adj_store && !adj_k[0])

@@ -1,0 +1,106 @@
+"""Device allocations that fail: a gradient, a descent and a demag plan go on
+with what the handle can hold.  A preloaded stand-in of cudaMalloc returns
+cudaErrorMemoryAllocation for requests above a limit that the child process
+sets; no memory is exhausted."""
+import os
+import subprocess
+import sys
+
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+PATHS = [ROOT, os.path.join(ROOT, "micromagnetic.jl_b200"), os.path.dirname(os.path.abspath(__file__))]
+
+SHIM = r"""
+#define _GNU_SOURCE
+#include <dlfcn.h>
+#include <stddef.h>
+static size_t limit = (size_t)-1;
+static long failed;
+void fake_limit(size_t n) { limit = n; }
+long fake_failed(void) { return failed; }
+int cudaMalloc(void** p, size_t n) {
+  static int (*real)(void**, size_t);
+  if (!real) real = (int (*)(void**, size_t))dlsym(dlopen("libcudart.so.12", RTLD_NOLOAD | RTLD_LAZY), "cudaMalloc");
+  if (n > limit) {
+    ++failed;
+    return 2;
+  }
+  return real(p, n);
+}
+"""
+
+HEAD = """
+import ctypes, sys
+sys.path[:0] = %r
+import numpy as np
+from helpers import GpuSim, random_config
+fake = ctypes.CDLL(None)
+fake.fake_limit.argtypes = [ctypes.c_size_t]
+fake.fake_failed.restype = ctypes.c_long
+""" % (PATHS,)
+
+
+@pytest.fixture(scope="module")
+def child(tmp_path_factory):
+    torch = pytest.importorskip("torch")
+    if not torch.cuda.is_available():
+        pytest.skip("no CUDA device")
+    d = tmp_path_factory.mktemp("fake_alloc")
+    (d / "shim.c").write_text(SHIM)
+    so = str(d / "shim.so")
+    subprocess.run(["gcc", "-shared", "-fPIC", "-O1", "-o", so, str(d / "shim.c"), "-ldl"], check=True)
+
+    def run(code, **env):
+        """Runs code with the fake in place; it leaves its results in the dict `out`."""
+        path = str(d / "out.npz")
+        r = subprocess.run([sys.executable, "-c", HEAD + code + f"\nnp.savez({path!r}, **out)\n"],
+                           env=dict(os.environ, LD_PRELOAD=so, **env), capture_output=True, text=True, timeout=600)
+        assert r.returncode == 0, r.stdout + r.stderr
+        return dict(np.load(path))
+
+    return run
+
+
+def close(a, b, tol):
+    assert np.max(np.abs(a - b)) <= tol * np.max(np.abs(b))
+
+
+GRAD = """
+cfg = random_config(3, 24, 20, 2, terms=("exch", "dmi_int", "anis", "demag"), holes=False)
+out = {}
+for limit in (2**62, 1 << 20):  # the segment's stage values take 2.5 MB
+    g = GpuSim(cfg, form=0)
+    g.h.call("mm_adjoint_record", 5e-14, 20, 10)
+    for call in range(3):
+        fake.fake_limit(limit)
+        o = [np.zeros(3 * g.n)] + [np.zeros(g.n) for _ in range(3)]
+        g.h.call("mm_adjoint_backward", g.lib.dptr(np.ones(3 * g.n)), *(g.lib.dptr(x) for x in o))
+        fake.fake_limit(2**62)
+        for k, x in enumerate(o):
+            out["%d_%d_%d" % (limit > 1 << 20, call, k)] = x
+    out["failed%d" % (limit > 1 << 20)] = np.array(fake.fake_failed())
+"""
+
+
+def test_gradient_without_room_for_stage_values(child):
+    """Both ways evaluate the same stages, the slopes by two kernels whose
+    roundings differ: 20 steps of FP64 agree to 1e-11."""
+    r = child(GRAD)
+    assert r["failed1"] == 0 and r["failed0"] == 3  # asked for again by every call
+    for call in range(3):
+        for k in range(4):
+            np.testing.assert_array_equal(r[f"0_{call}_{k}"], r[f"0_0_{k}"])
+            close(r[f"0_{call}_{k}"], r[f"1_{call}_{k}"], 1e-11)
+
+
+@pytest.mark.parametrize("env", [{"MMCUDA_ADJ_STORE": "0"}])
+def test_gradient_keeps_no_stage_values(child, env):
+    """Switched off."""
+    a, b = child(GRAD, **env), child(GRAD)
+    for call in range(3):
+        for k in range(4):
+            close(a[f"1_{call}_{k}"], b[f"1_{call}_{k}"], 1e-11)
