@@ -65,13 +65,21 @@ __global__ void k_to_double(const R* __restrict__ a, double* __restrict__ b, int
   if (i < n) b[i] = static_cast<double>(a[i]);
 }
 
-// MMCUDA_ADJ_STORE=0: gradients keep no stage values
+// MMCUDA_ADJ_STORE=0: gradients keep no stage values; MMCUDA_ADJ_KEEP_MB: the
+// size up to which a handle keeps them between calls (1024)
 static bool adj_store_enabled() {
   static const bool on = [] {
     const char* e = getenv("MMCUDA_ADJ_STORE");
     return !(e && e[0] == '0');
   }();
   return on;
+}
+static size_t adj_keep_bytes() {
+  static const size_t v = [] {
+    const char* e = getenv("MMCUDA_ADJ_KEEP_MB");
+    return static_cast<size_t>(e ? std::max(0, atoi(e)) : 1024) << 20;
+  }();
+  return v;
 }
 
 class EngineBase {
@@ -1378,7 +1386,7 @@ class Engine : public EngineBase {
       for (int64_t s = len - 1; s >= 0; --s)
         adj_step_back(adj_seg + s * n3, kF32 ? adj_seg_lo + s * n3 : nullptr, adj_dt, s);
     };
-    if (adj_calls == 0 || len > 64) {
+    if (adj_calls == 0 || len > 64 || sizeof(R) * kAdjVecs * 3 * N * adj_store_cap > adj_keep_bytes()) {
       enqueue();
       MM_CUDA(cudaGetLastError());
       return MM_OK;
@@ -1415,7 +1423,21 @@ class Engine : public EngineBase {
     }
   }
 
+  // Stage values beyond 1 GiB are held for the call only (a handle that keeps
+  // many GB between calls starves the others of the device; at that size an
+  // allocation and the segments' launches cost nothing beside the kernels).
   int adjoint_backward(const double* dLdm, double* gm0, double* gMs, double* gKu, double* gD) override {
+    const int rc = adj_backward(dLdm, gm0, gMs, gKu, gD);
+    if (sizeof(R) * kAdjVecs * 3 * N * adj_store_cap > adj_keep_bytes()) {
+      cudaStreamSynchronize(st_);
+      adj_drop_graphs();
+      release(adj_store, adj_store_cap * kAdjVecs * 3 * N);
+      adj_store_cap = 0;
+    }
+    return rc;
+  }
+
+  int adj_backward(const double* dLdm, double* gm0, double* gMs, double* gKu, double* gD) {
     if (!adj_n) return fail(MM_ERR_STATE, "mm_adjoint_record must run first");
     if (adj_version != version) return fail(MM_ERR_STATE, "parameters changed since mm_adjoint_record");
     if (!dLdm) return fail(MM_ERR_ARG, "null dL/dm");

@@ -97,10 +97,29 @@ def test_gradient_without_room_for_stage_values(child):
             close(r[f"0_{call}_{k}"], r[f"1_{call}_{k}"], 1e-11)
 
 
-@pytest.mark.parametrize("env", [{"MMCUDA_ADJ_STORE": "0"}])
+@pytest.mark.parametrize("env", [{"MMCUDA_ADJ_STORE": "0"}, {"MMCUDA_ADJ_KEEP_MB": "0"}])
 def test_gradient_keeps_no_stage_values(child, env):
-    """Switched off."""
+    """Switched off, and given back after every call."""
     a, b = child(GRAD, **env), child(GRAD)
     for call in range(3):
         for k in range(4):
             close(a[f"1_{call}_{k}"], b[f"1_{call}_{k}"], 1e-11)
+
+
+BYTES = """
+cfg = random_config(3, 24, 20, 2, terms=("exch", "dmi_int", "anis", "demag"), holes=False)
+g = GpuSim(cfg, form=0)
+out = {"b": []}
+for call in range(4):
+    g.h.call("mm_adjoint_record", 5e-14, 20, 10)
+    o = [np.zeros(3 * g.n)] + [np.zeros(g.n) for _ in range(3)]
+    g.h.call("mm_adjoint_backward", g.lib.dptr(np.ones(3 * g.n)), *(g.lib.dptr(x) for x in o))
+    out["b"].append(g.h.device_bytes())
+"""
+
+
+def test_large_stage_values_are_given_back(child):
+    """Above the kept size a handle holds the values during the call only."""
+    kept, given = child(BYTES)["b"], child(BYTES, MMCUDA_ADJ_KEEP_MB="0")["b"]
+    assert len(set(kept)) == 1 and len(set(given)) == 1
+    assert kept[0] - given[0] == 8 * 11 * 3 * 960 * 10
