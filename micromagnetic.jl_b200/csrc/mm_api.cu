@@ -1152,15 +1152,17 @@ class Engine : public EngineBase {
       const bool dm = (mask & TB_DEMAG) && demag;
       DemagPlan<R>* const plan = dm ? sd_plan() : nullptr;
       if (dm && !plan) return MM_ERR_CUDA;
-      // iterations are enqueued up to eight at a time; past the stopping one their
-      // kernels return at once
+      // iterations are enqueued one, four and then eight at a time (a descent that
+      // has converged already pays for one); past the stopping one their kernels
+      // return at once
       int64_t queued = 0;
-      while (hs.active && queued < max_steps) {
-        for (int q = 0; q < 8 && queued < max_steps; ++q, ++queued) {
-          enqueue_thermal(th_step, nullptr, th_dt, nullptr);
+      for (int group = 1; hs.active && queued < max_steps; group = std::min(8, 4 * group)) {
+        for (int q = 0; q < group && queued < max_steps; ++q, ++queued) {
+          enqueue_thermal(th_step, nullptr, th_dt, &sd->active);
           if (plan) plan->apply(m, Ms, Hd, st_, &sd->active, plan->runtime_ok && !kF32);
           StageArgs<R> sf{};
           sf.out = work;
+          sf.gate = &sd->active;
           launch_stage<R>(SM_FIELD, fargs(~0u), m, sf, st_);
           launch_sd_gk<R>(m, pre, work, gk, N, sd_steps == 0 ? 1 : 0, partials, sd, st_);
           launch_sd_tau(sd, partials, nb, st_);

@@ -132,6 +132,7 @@ template <typename R> struct StageArgs {
   int scheme;               // fixed-step scheme: 0 RK4, 1 Heun (modified Euler)
   int method;               // SM_DOPRI: RkMethod
   const DopriCtrl* ctrl;    // SM_DOPRI: step size and active flag
+  const int* gate;          // SM_FIELD: the kernel returns at once when *gate == 0 (null: always runs)
 };
 
 template <typename R>

@@ -390,6 +390,7 @@ void launch_zsmall_pz(const DemagGeom& g, cplx_t<R>* Y, const R* Nhat, cudaStrea
   typename ZSmall<R, PZ>::Args a{};
   a.Y = Y;
   a.Nhat = Nhat;
+  a.gate = g.gate;
   a.Hx = g.Hx;
   a.Py = g.Py;
   a.nz = g.nz;

@@ -560,12 +560,14 @@ struct ZSmall {
   struct Args {
     cplx_t<R>* Y;
     const R* __restrict__ Nhat;
+    const int* gate;  // device flag: return at once when *gate == 0 (null: always run)
     int Hx, Py, nz, Tyq, Tzq;
     R twr[PZ], twi[PZ];  // w^t = exp(-2 pi i t / PZ)
     dim3 grid;
   };
   static __device__ __forceinline__ void body(const Args& a, uint3 blockIdx) {
     using C = cplx_t<R>;
+    if (a.gate && !*a.gate) return;
     const int64_t line = static_cast<int64_t>(blockIdx.x) * kNT + threadIdx.x;
     const int Hx = a.Hx, Py = a.Py, nz = a.nz;
     if (line >= static_cast<int64_t>(Hx) * Py) return;

@@ -51,6 +51,7 @@ __global__ void __launch_bounds__(kStageThreads, sizeof(R) == 4 ? 3 : 2) k_stage
   constexpr bool kF32 = sizeof(R) == 4;
   pdl_enter();
   if (MODE == SM_DOPRI && !s.ctrl->active) return;
+  if (MODE == SM_FIELD && s.gate && !*s.gate) return;
   const int64_t N = a.N;
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   const int j = blockIdx.y * blockDim.y + threadIdx.y;
