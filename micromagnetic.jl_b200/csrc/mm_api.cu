@@ -500,14 +500,22 @@ class Engine : public EngineBase {
   // stopping criterion is met moves by a third), so a descent keeps the
   // arithmetic its earlier results came from.  Where the compile-time lengths
   // differ from the run-time ones the second plan is built at the first
-  // descent.  Nullptr on failure.
+  // descent (its tensor is assembled again, and its buffers stay with the
+  // handle); without room for it the descent runs on the handle's own plan.
+  // The rule keeps published relaxations as they were (standard problem 4: the
+  // step count is compared with the oracle's); it makes no descent safer.  FP64
+  // boxes and the FP32 form follow the handle's plan: their trajectories equal
+  // earlier ones up to the same amplified rounding.
   DemagPlan<R>* sd_plan() {
     if (!demag || kF32 || nz > 1 || !demag->rfft || demag->runtime_ok) return demag.get();
     if (!demag_sd) {
       auto p = std::make_unique<DemagPlan<R>>();
-      if (build_demag(*p, images_[0], images_[1], images_[2], tensor_.empty() ? nullptr : tensor_.data(), true))
-        return nullptr;
+      if (build_demag(*p, images_[0], images_[1], images_[2], tensor_.empty() ? nullptr : tensor_.data(), true)) {
+        cudaGetLastError();
+        return demag.get();
+      }
       demag_sd = std::move(p);
+      std::vector<double>().swap(tensor_);
     }
     return demag_sd.get();
   }
@@ -1149,9 +1157,7 @@ class Engine : public EngineBase {
       SdState hs{0.0, 1.0, 1e-10, sd_steps, 0.0, stop * dmdt_factor, 0, 1};
       MM_CUDA(cudaMemcpyAsync(sd, &hs, sizeof(hs), cudaMemcpyHostToDevice, st_));
       const int nb = stage_blocks(N);
-      const bool dm = (mask & TB_DEMAG) && demag;
-      DemagPlan<R>* const plan = dm ? sd_plan() : nullptr;
-      if (dm && !plan) return MM_ERR_CUDA;
+      DemagPlan<R>* const plan = (mask & TB_DEMAG) && demag ? sd_plan() : nullptr;
       // iterations are enqueued one, four and then eight at a time (a descent that
       // has converged already pays for one); past the stopping one their kernels
       // return at once

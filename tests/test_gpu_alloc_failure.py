@@ -123,3 +123,31 @@ def test_large_stage_values_are_given_back(child):
     kept, given = child(BYTES)["b"], child(BYTES, MMCUDA_ADJ_KEEP_MB="0")["b"]
     assert len(set(kept)) == 1 and len(set(given)) == 1
     assert kept[0] - given[0] == 8 * 11 * 3 * 960 * 10
+
+
+DESCENT = """
+from oracle.oracle import demag_tensor
+cfg = random_config(5, 101, 97, 1, terms=("exch", "anis", "demag"))
+T = demag_tensor(101, 97, 1, cfg["dx"], cfg["dy"], cfg["dz"])
+out = {}
+for name, tensor in (("own", None), ("given", T)):
+    for limit in (2**62, 300000):  # the second plan's spectra take 475 kB
+        g = GpuSim(cfg, form=0, tensor=tensor)
+        n, mx = ctypes.c_int64(), ctypes.c_double()
+        for part in (2, 2):
+            fake.fake_limit(limit)
+            g.h.call("mm_relax", 0, part, 0.0, ctypes.byref(n), ctypes.byref(mx))
+            fake.fake_limit(2**62)
+        out["%s%d" % (name, limit < 2**62)] = g.m()
+    out["failed_" + name] = np.array(fake.fake_failed())
+"""
+
+
+def test_descent_without_room_for_its_own_plan(child):
+    """An FP64 film's descent takes the handle's own plan when its second one
+    cannot be allocated.  The first steps: the step lengths have not yet
+    amplified the rounding (1e-15) of the two transforms beyond 1e-11."""
+    r = child(DESCENT)
+    assert r["failed_own"] > 0 and r["failed_given"] > r["failed_own"]
+    for name in ("own", "given"):
+        close(r[name + "1"], r[name + "0"], 1e-11)
