@@ -524,7 +524,14 @@ class Engine : public EngineBase {
     if (mask & TB_DEMAG) return fail(MM_ERR_UNSUPPORTED, "one demag term per handle");
     if (Nx < 0 || Ny < 0 || Nz < 0) return fail(MM_ERR_ARG, "macro-PBC image counts must be >= 0");
     auto plan = std::make_unique<DemagPlan<R>>();
-    if (int rc = build_demag(*plan, Nx, Ny, Nz, T6N_host, false)) return rc;
+    if (int rc = build_demag(*plan, Nx, Ny, Nz, T6N_host, false)) {
+      if (!plan->rfft) return rc;
+      // the compile-time lengths pad more (up to a third more spectrum): a mesh
+      // that does not fit with them may with the run-time ones
+      cudaGetLastError();
+      plan = std::make_unique<DemagPlan<R>>();
+      if ((rc = build_demag(*plan, Nx, Ny, Nz, T6N_host, true))) return rc;
+    }
     images_[0] = Nx; images_[1] = Ny; images_[2] = Nz;
     // a tensor of the caller's is kept where a descent may need it again (sd_plan)
     if (T6N_host && !kF32 && nz == 1 && plan->rfft && !plan->runtime_ok) tensor_.assign(T6N_host, T6N_host + 6 * N);

@@ -855,13 +855,15 @@ bool DemagPlan<R>::launch_pass(int which, const R* m, const R* mu0Ms, R* Hd, cud
 // For each strided pass the plan uses, time every valid tile width W (powers
 // of two up to a 128-byte row segment, within the 200 KB shared-memory limit
 // and, for the fused-middle z kernel, W * RA <= threads) on the plan's own
-// buffers and keep the fastest.  Results are cached per (form, mesh shape),
-// so a batch of equal meshes tunes once.  MMCUDA_AUTOTUNE=0 keeps the static
+// buffers and keep the fastest.  Results are cached per (form, kind of
+// lengths, mesh shape), so a batch of equal meshes tunes once.  MMCUDA_AUTOTUNE=0 keeps the static
 // rule.
 struct TileKey {
-  int w, nx, ny, nz;
+  int w;
+  bool rfft;
+  int nx, ny, nz;
   bool operator<(const TileKey& o) const {
-    return std::tie(w, nx, ny, nz) < std::tie(o.w, o.nx, o.ny, o.nz);
+    return std::tie(w, rfft, nx, ny, nz) < std::tie(o.w, o.rfft, o.nx, o.ny, o.nz);
   }
 };
 static std::mutex g_tile_mu;
@@ -872,7 +874,7 @@ int DemagPlan<R>::autotune(const R* m, const R* mu0Ms, R* Hd, cudaStream_t st) {
   using C = cplx_t<R>;
   const char* env = getenv("MMCUDA_AUTOTUNE");
   if (env && env[0] == '0') return 0;
-  const TileKey key{static_cast<int>(sizeof(R)), g.nx, g.ny, g.nz};
+  const TileKey key{static_cast<int>(sizeof(R)), rfft, g.nx, g.ny, g.nz};
   {
     std::lock_guard<std::mutex> lk(g_tile_mu);
     auto it = g_tile_cache.find(key);

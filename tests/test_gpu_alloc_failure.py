@@ -151,3 +151,31 @@ def test_descent_without_room_for_its_own_plan(child):
     assert r["failed_own"] > 0 and r["failed_given"] > r["failed_own"]
     for name in ("own", "given"):
         close(r[name + "1"], r[name + "0"], 1e-11)
+
+
+PLAN = """
+cfg = random_config(4, 8, 13, 128, terms=("exch", "demag"))
+out = {}
+for form in (0, 1):
+    w = 4 if form else 8
+    GpuSim(cfg, form=form).h.close()  # the tile widths kept for this mesh are those of the other lengths
+    fake.fake_limit(250000 * w)  # y spectrum: 1.20 MB (FP32) at the compile-time lengths, 0.69 at the others
+    f = fake.fake_failed()
+    g = GpuSim(cfg, form=form)
+    fake.fake_limit(2**62)
+    out["failed%d" % form] = np.array(fake.fake_failed() - f)
+    out["field%d" % form] = g.field()
+"""
+
+
+def test_demag_without_room_for_the_longer_lines(child):
+    """The compile-time lengths pad more; where their buffers do not fit, the
+    plan takes the run-time lengths."""
+    from helpers import build_oracle, random_config, rel_maxnorm
+
+    r = child(PLAN)
+    o, _ = build_oracle(random_config(4, 8, 13, 128, terms=("exch", "demag")))
+    ref = o.effective_field()
+    for form, tol in ((0, 1e-12), (1, 1e-5)):
+        assert r[f"failed{form}"] > 0
+        assert rel_maxnorm(r[f"field{form}"], ref) <= tol
