@@ -774,6 +774,7 @@ class Engine : public EngineBase {
     if (!persist_.ready() || ps_dt != dt || ps_version != version) {
       std::vector<std::vector<LaunchRec>> recs(1);
       LaunchRecorder rec;
+      rec.persist = true;
       launch_recorder() = &rec;
       enqueue_rk4_step(dt);
       launch_recorder() = nullptr;
@@ -1960,6 +1961,7 @@ int mm_batch_rk4_run(mm_batch* b, double dt, int64_t nsteps) {
         std::vector<std::vector<mm::LaunchRec>> recs(n);
         for (int i = 0; i < n; ++i) {
           mm::LaunchRecorder rec;
+          rec.persist = true;
           mm::launch_recorder() = &rec;
           b->hs[i]->eng->rk4_enqueue(dt);
           mm::launch_recorder() = nullptr;

@@ -184,8 +184,10 @@ void launch_stage(int mode, const FieldArgs<R>& fa, const R* y, const StageArgs<
                            {fa, y, sa, static_cast<int>(g.block.x), static_cast<int>(g.block.y), dim3()});
     return;
   }
-  // MMCUDA_STAGE_FIX=0 keeps the general kernel
-  const bool uni = !fa.A && !fa.D && !fa.Ku && !fa.Hz && stage_fix_enabled();
+  // MMCUDA_STAGE_FIX=0 keeps the general kernel, as the persistent step does (it
+  // has that form only)
+  const LaunchRecorder* const rec = launch_recorder();
+  const bool uni = !fa.A && !fa.D && !fa.Ku && !fa.Hz && stage_fix_enabled() && !(rec && rec->persist);
   if (mode == SM_RK4) {
     if (uni && launch_rk4_fix<R>(fa, y, sa, g, st)) return;
     launch_k<StagePlain<R>>(g.grid, 0, st, {fa, y, sa, static_cast<int>(g.block.x), static_cast<int>(g.block.y), dim3()});

@@ -79,6 +79,7 @@ struct LaunchRec {
 
 struct LaunchRecorder {
   std::vector<LaunchRec> recs;
+  bool persist = false;  // for the persistent step kernel: only kernels that have a form in it
 };
 LaunchRecorder*& launch_recorder();  // the calling thread's active recorder (null: launch)
 // Raises the dynamic shared-memory limit of a kernel to the opt-in maximum,

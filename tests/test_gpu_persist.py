@@ -114,3 +114,40 @@ def test_barrier_wait_limit_reports_timeout(tmp_path):
     r = _child(TIMEOUT, {"MMCUDA_PERSIST": "1", "MMCUDA_BARRIER_SPINS": "1"}, tmp_path)
     assert r.returncode == 0, r.stdout + r.stderr
     assert "rc -5" in r.stdout and "grid-barrier" in r.stdout, r.stdout
+
+
+UNIFORM = """
+import numpy as np
+from helpers import GpuSim, random_config
+from mmcuda import _lib
+out = {}
+for k, terms in enumerate(%r):
+    sims = []
+    for mesh in ((40, 24, 1, ""), (33, 17, 1, "")):
+        cfg = random_config(9 + mesh[0], *mesh, terms=terms, spatial=False)
+        cfg["H"] = np.tile([2e4, -1e4, 3e4], cfg["Ms"].size)
+        sims.append(GpuSim(cfg, form=1))
+    b = _lib.Batch([s.h for s in sims])
+    b.rk4_run(2e-14, 5)
+    out["launches%%d" %% k] = np.array(b.launches())
+    for j, s in enumerate(sims):
+        out["m%%d_%%d" %% (k, j)] = s.m()
+    b.close()
+np.savez(%r, **out)
+"""
+
+
+def test_uniform_parameters_run_persistently(tmp_path):
+    """Term sets with uniform parameters have compiled stage kernels, which the
+    persistent step does not hold: it takes the general form of the stage."""
+    sets = [("exch", "demag"), ("exch", "anis", "demag"), ("exch", "dmi_int", "anis", "zeeman", "demag"),
+            ("exch", "dmi_bulk", "zeeman", "demag")]
+    paths = [str(tmp_path / f"u{flag}.npz") for flag in "01"]
+    for flag, path in zip("01", paths):
+        r = _child(UNIFORM % (sets, path), {"MMCUDA_PERSIST": flag}, tmp_path)
+        assert r.returncode == 0, r.stdout + r.stderr
+    plain, persist = (np.load(p) for p in paths)
+    for k in range(len(sets)):
+        assert tuple(persist[f"launches{k}"]) == (1, 2) and plain[f"launches{k}"][0] > 1
+        for j in range(2):
+            assert rel_maxnorm(persist[f"m{k}_{j}"], plain[f"m{k}_{j}"]) <= 1e-6
