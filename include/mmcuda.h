@@ -230,6 +230,9 @@ int mm_add_thermal_noise(mm_handle* h, const double* T, double T_uniform, double
  * (N, uniaxial anisotropy) and dL/dD per cell (N, interfacial DMI; for a
  * uniform D the scalar gradient is the sum).  Segments of ckpt_every steps
  * are recomputed forward (3N*ckpt_every state words kept); m is left at m_T.
+ * Where it takes at most a quarter of the free device memory the stage values
+ * of a segment (33N*ckpt_every words) are kept too, beyond 1 GiB for the call
+ * only; without them every stage is evaluated once more.
  * Changing parameters between the two calls is refused (MM_ERR_STATE). */
 int mm_adjoint_record(mm_handle* h, double dt, int64_t nsteps, int64_t ckpt_every);
 int mm_adjoint_backward(mm_handle* h, const double* dL_dmT, double* g_m0, double* g_Ms, double* g_Ku, double* g_D);
@@ -253,7 +256,11 @@ int mm_save_ovf(mm_handle* h, const char* path, int type, const char* title);
 int mm_load_ovf(mm_handle* h, const char* path);
 
 /* relax(sim; max_steps, stopping_dmdt)  src/sim.jl:392-490 with the SD
- * driver (src/sd.jl:9-98) or the LLG driver with Dormand-Prince */
+ * driver (src/sd.jl:9-98) or the LLG driver with Dormand-Prince.  The first
+ * descent (SD) of an FP64 film of 8192 cells and more whose padded lengths
+ * differ between the two kinds of FFT passes builds a second demag plan: the
+ * cost of mm_add_demag once more, and its memory until the handle is destroyed
+ * (the handle's own plan serves when there is no room). */
 int mm_relax(mm_handle* h, int driver, int64_t max_steps, double stopping_dmdt, int64_t* steps_done,
              double* max_dmdt);
 

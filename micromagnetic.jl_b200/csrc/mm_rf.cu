@@ -1,4 +1,6 @@
 // mm_rf.cu -- host-side length rules of the compile-time FFT passes.
+#include <algorithm>
+
 #include "mm_rf.cuh"
 #include "mm_rfpass.cuh"
 
@@ -44,6 +46,24 @@ template <int L> constexpr Entry entry() {
 constexpr Entry kEntries[] = {MM_RF_LENGTHS_A(E) MM_RF_LENGTHS_B(E) MM_RF_LENGTHS_C(E) MM_RF_LENGTHS_D(E)
                                   MM_RF_LENGTHS_E(E) MM_RF_LENGTHS_F(E) MM_RF_LENGTHS_G(E)};
 #undef E
+
+// largest padding of the next length over a request between lo and hi, in 1/1000
+constexpr int worst_padding(Kind k, bool f64, int lo, int hi) {
+  int worst = 0, prev = 0;
+  for (const Entry& e : kEntries) {
+    if (!e.w[f64][k]) continue;
+    if (prev >= lo && e.L <= hi) worst = std::max(worst, (1000 * e.L + prev) / (prev + 1) - 1000);
+    prev = e.L;
+  }
+  return worst;
+}
+constexpr bool padding_bounded() {
+  for (Kind k : {KX, KY, KZ, KC})
+    for (bool f64 : {false, true})
+      if (worst_padding(k, f64, 100, 4096) > 125 || worst_padding(k, f64, 12, 100) > 231) return false;
+  return true;
+}
+static_assert(padding_bounded(), "the lengths leave gaps above 12.5 % (23 % below 100 points)");
 }  // namespace
 
 int next_length(Kind k, bool f64, int n) {

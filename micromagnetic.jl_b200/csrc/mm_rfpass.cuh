@@ -458,9 +458,9 @@ template <typename R> constexpr bool z_has(int L) { return L <= 256 && radices(L
 // column is one contiguous run of memory.
 // SPLIT (columns beyond 4096, one block an SM): the last stage, the product and
 // the first inverse stage as three passes over shared memory instead of 3 R3
-// values in registers, so that the block has 600 threads instead of 400 (the
-// 8000-point columns of a 4000 x 4000 film, where 13 warps issued on 41 % of the
-// cycles: 868 -> 734 us).
+// values in registers, so that the block has 3/2 threads a butterfly (8000-point
+// columns: 600 instead of 400 threads; 4000 x 4000 film, where 13 warps issued on
+// 41 % of the cycles: 868 -> 734 us).
 template <typename R, int L> struct FilmConv {
   using P = Plan<R, L, cap3(sizeof(R) == 8, L)>;
   using C = typename P::C;
