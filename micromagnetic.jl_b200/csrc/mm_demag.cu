@@ -264,25 +264,43 @@ void smem_optin(const void* kernel) {
   done.insert({kernel, dev});
 }
 
-// exp(-2 pi i t / L), t < L; Q > 0 (L = 64 Q, the register passes): followed by
-// their table exp(-2 pi i q k / (L / 2)) at k Q + q, k < 32, q < Q
-template <typename C>
-static C* upload_twiddles(int L, size_t& bytes, cudaStream_t st, int Q = 0) {
+// exp(-2 pi i t / L)
+template <typename C> static C unit_root(int64_t t, int L) {
+  const long double a = -2.0L * 3.141592653589793238462643383279502884L * static_cast<long double>(t) / L;
+  C c;
+  c.x = static_cast<decltype(C::x)>(static_cast<double>(cosl(a)));
+  c.y = static_cast<decltype(C::x)>(static_cast<double>(sinl(a)));
+  return c;
+}
+
+// exp(-2 pi i t / L), t < L
+template <typename C> static std::vector<C> twiddle_table(int L) {
   std::vector<C> h(L);
-  for (int t = 0; t < L; ++t) {
-    const long double a = -2.0L * 3.141592653589793238462643383279502884L * t / L;
-    h[t].x = static_cast<decltype(C::x)>(static_cast<double>(cosl(a)));
-    h[t].y = static_cast<decltype(C::x)>(static_cast<double>(sinl(a)));
-  }
-  for (int k = 0; k < (Q > 0 ? 32 : 0); ++k)
-    for (int q = 0; q < Q; ++q) h.push_back(h[2 * q * k]);
-  const int n = static_cast<int>(h.size());
+  for (int t = 0; t < L; ++t) h[t] = unit_root<C>(t, L);
+  return h;
+}
+
+template <typename C> static C* upload_table(const std::vector<C>& h, size_t& bytes, cudaStream_t st) {
+  const size_t n = sizeof(C) * h.size();
   C* d = nullptr;
-  if (cudaMalloc(&d, sizeof(C) * n) != cudaSuccess) return nullptr;
-  bytes += sizeof(C) * n;
-  cudaMemcpyAsync(d, h.data(), sizeof(C) * n, cudaMemcpyHostToDevice, st);
+  if (cudaMalloc(&d, n) != cudaSuccess) return nullptr;
+  bytes += n;
+  cudaMemcpyAsync(d, h.data(), n, cudaMemcpyHostToDevice, st);
   cudaStreamSynchronize(st);
   return d;
+}
+
+// the table of length L; Q > 0 (L = 64 Q, the register passes): followed by
+// their table exp(-2 pi i q k / (L / 2)) at k Q + q, k < 32, q < Q
+template <typename C>
+static C* upload_twiddles(std::vector<C> h, size_t& bytes, cudaStream_t st, int Q = 0) {
+  for (int k = 0; k < (Q > 0 ? 32 : 0); ++k)
+    for (int q = 0; q < Q; ++q) h.push_back(C(h[2 * q * k]));
+  return upload_table(h, bytes, st);
+}
+template <typename C>
+static C* upload_twiddles(int L, size_t& bytes, cudaStream_t st) {
+  return upload_table(twiddle_table<C>(L), bytes, st);
 }
 
 template <typename R>
@@ -314,23 +332,19 @@ static bool rfft_enabled() {
 // bound by launches either way.
 constexpr int64_t kRfftCells = 8192;
 
-// tw2[(r-1) R1 + k] = w_{R1 R2}^(r k), tw3[(q-1) R1 R2 + i] = w_L^(q i)
+// tw2[(r-1) R1 + k] = w_{R1 R2}^(r k), tw3[(q-1) R1 R2 + i] = w_L^(q i), from
+// the plan's table of length step L (sines of their own took 0.25 ms of the 5.5
+// ms that add_demag takes for a 1000 x 1000 film)
 template <typename C>
-static void fill_rf_twiddles(const rf::Radices& f, std::vector<C>& out, size_t& o2, size_t& o3) {
+static void fill_rf_twiddles(const rf::Radices& f, const std::vector<C>& table, int step, std::vector<C>& out, size_t& o2,
+                             size_t& o3) {
   const int L = f.r1 * f.r2 * f.r3, M = f.r1 * f.r2;
-  auto push = [&](int64_t num, int den) {
-    const long double a = -2.0L * 3.141592653589793238462643383279502884L * static_cast<long double>(num % den) / den;
-    C c;
-    c.x = static_cast<decltype(C::x)>(static_cast<double>(cosl(a)));
-    c.y = static_cast<decltype(C::x)>(static_cast<double>(sinl(a)));
-    out.push_back(c);
-  };
   o2 = out.size();
   for (int r = 1; r < f.r2; ++r)
-    for (int k = 0; k < f.r1; ++k) push(static_cast<int64_t>(r) * k, M);
+    for (int k = 0; k < f.r1; ++k) out.push_back(unit_root<C>(r * k % M, M));
   o3 = out.size();
   for (int q = 1; q < f.r3; ++q)
-    for (int i = 0; i < M; ++i) push(static_cast<int64_t>(q) * i, L);
+    for (int i = 0; i < M; ++i) out.push_back(table[static_cast<int64_t>(q) * i % L * step]);
 }
 
 template <typename R>
@@ -453,19 +467,17 @@ int DemagPlan<R>::init(int nx, int ny, int nz, cudaStream_t st, char* err, size_
       return -1;
     }
   }
-  if (g.Px > 1 && !(twx = upload_twiddles<C>(g.Px, bytes_, st, g.wreg ? nx / 32 : 0))) return 2;
-  if (!(twy = upload_twiddles<C>(g.Py, bytes_, st, g.wreg ? ny / 32 : 0))) return 2;
-  if (!(twz = upload_twiddles<C>(g.Pz, bytes_, st))) return 2;
+  const std::vector<C> hx = twiddle_table<C>(g.Px), hy = twiddle_table<C>(g.Py), hz = twiddle_table<C>(g.Pz);
+  if (g.Px > 1 && !(twx = upload_twiddles<C>(hx, bytes_, st, g.wreg ? nx / 32 : 0))) return 2;
+  if (!(twy = upload_twiddles<C>(hy, bytes_, st, g.wreg ? ny / 32 : 0))) return 2;
+  if (!(twz = upload_twiddles<C>(hz, bytes_, st))) return 2;
   if (rfft) {
     std::vector<C> h;
     size_t o[6] = {};
-    fill_rf_twiddles(rf::plan_of(rf::KX, f64, g.Lc), h, o[0], o[1]);
-    fill_rf_twiddles(rf::plan_of(fused2d ? rf::KC : rf::KY, f64, g.Py), h, o[2], o[3]);
-    if (rfft_z) fill_rf_twiddles(rf::plan_of(rf::KZ, f64, g.Pz), h, o[4], o[5]);
-    if (cudaMalloc(&rtab, sizeof(C) * h.size()) != cudaSuccess) return 2;
-    bytes_ += sizeof(C) * h.size();
-    cudaMemcpyAsync(rtab, h.data(), sizeof(C) * h.size(), cudaMemcpyHostToDevice, st);
-    cudaStreamSynchronize(st);
+    fill_rf_twiddles(rf::plan_of(rf::KX, f64, g.Lc), hx, 2, h, o[0], o[1]);  // Px = 2 Lc
+    fill_rf_twiddles(rf::plan_of(fused2d ? rf::KC : rf::KY, f64, g.Py), hy, 1, h, o[2], o[3]);
+    if (rfft_z) fill_rf_twiddles(rf::plan_of(rf::KZ, f64, g.Pz), hz, 1, h, o[4], o[5]);
+    if (!(rtab = upload_table(h, bytes_, st))) return 2;
     rtx = {rtab + o[0], rtab + o[1]};
     rty = {rtab + o[2], rtab + o[3]};
     rtz = {rtab + o[4], rtab + o[5]};
