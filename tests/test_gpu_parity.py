@@ -113,11 +113,11 @@ def test_demag_long_lines(mesh, form):
 @pytest.mark.parametrize("form", [0, 1])
 @pytest.mark.parametrize("mesh", [(100, 80, 1), (40, 600, 1), (24, 1300, 1), (6, 2400, 1)])
 def test_film_paths(mesh, form):
-    """The film paths by column length (padded y = 160, 1200, 2600, 4800):
-    the fused column-major y convolution within the tile budget or filling one
-    block (FP64 y = 1200, FP32 y = 2600), and the global-memory y stages for
-    columns that fit no block (FP64 y = 2600, both forms at y = 4800); field
-    and two RK4 steps against the oracle."""
+    """The film paths: columns in one block on compile-time lengths (padded
+    y = 1200, 2700), and for the smaller and the narrow film the run-time passes
+    (y = 160, and 4800 in global-memory stages); field and two RK4 steps against
+    the oracle.  test_run_time_passes_against_oracle holds the run-time passes of
+    the other columns."""
     from oracle.oracle import demag_tensor
 
     nx, ny, nz = mesh
