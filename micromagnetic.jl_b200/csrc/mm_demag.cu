@@ -327,9 +327,11 @@ static bool rfft_enabled() {
   }();
   return on && !persist_enabled();
 }
-// Smaller meshes keep the run-time-length passes: their kernels are the same
-// for every length, so a batch of them shares launches, and one such mesh is
-// bound by launches either way.
+// Smaller meshes keep the run-time-length passes: their kernels are the same for
+// every length, so a batch of uneven ones is a few merged launches.  The line is
+// not the fastest one: with it at 64 cells a step of a 64 x 64 film took 45 us
+// instead of 66 (FP32; 51 and 59 in FP64), and 32 films of 24 to 60 cells a side
+// 0.14 ms in 352 launches instead of 0.22 in 16.
 constexpr int64_t kRfftCells = 8192;
 
 // tw2[(r-1) R1 + k] = w_{R1 R2}^(r k), tw3[(q-1) R1 R2 + i] = w_L^(q i), from
