@@ -1,7 +1,7 @@
 // mm_oracle.cpp -- CPU FP64 restatement of the MicroMagnetic.jl finite-difference
 // hot path (effective field, LLG right-hand side, RK4 / Dormand-Prince, SD relax).
 //
-// TEST INFRASTRUCTURE ONLY.  This file is the checker: it is loaded by tests/,
+// TEST INFRASTRUCTURE ONLY.  Results are compared with it: it is loaded by tests/,
 // by __graft_entry__.smoke() and by bench.py's CPU-baseline leg.  The product
 // library (libmmcuda.so) never links, loads or calls it.
 //

@@ -1,7 +1,7 @@
 """ctypes wrapper of the CPU FP64 oracle (``mm_oracle.cpp``).
 
 TEST INFRASTRUCTURE ONLY: imported by ``tests/``, by ``__graft_entry__.smoke()``
-and by ``bench.py``'s CPU-baseline leg, as the checker.  The product package
+and by ``bench.py``'s CPU-baseline leg to compare with.  The product package
 never imports it.
 
 The oracle restates the MicroMagnetic.jl finite-difference path (see the
