@@ -103,8 +103,8 @@ def test_c1_film_inplane_zeeman():
 
 
 def test_c2_bulk_rk4():
-    """256x256x64: exchange, bulk DMI, anisotropy, demag (row-major z tiles
-    with leftover kx columns)."""
+    """256x256x64: exchange, bulk DMI, anisotropy, demag (y lines of 512, z lines
+    of 128 points)."""
     _check_workload("c2", steps=(1,))
 
 
@@ -205,8 +205,8 @@ def _film_oracle(s):
 
 
 def test_c3_films_including_odd_padding():
-    """Films of the c3 set plus nx = 251 (7-smooth padding 504 here, 502 in
-    the oracle) and ny = 251: H_eff and one RK4 step each."""
+    """Films of the c3 set plus nx = 251 (padded to 512 here, 502 in the oracle)
+    and ny = 251: H_eff and one RK4 step each."""
     from mmcuda import _lib
 
     specs = bench.batch_specs("c3")

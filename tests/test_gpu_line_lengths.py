@@ -66,8 +66,11 @@ np.savez(%r, **out)
 """
 # film columns within the tile budget, filling one block (FP64 1200, FP32 2600
 # points) and in global-memory stages (FP64 2600); leftover columns of a
-# power-of-two z convolution; other z lengths; wide and narrow row tiles
-RUNTIME_MESHES = [(100, 82, 1), (40, 600, 1), (24, 1300, 1), (64, 10, 16), (97, 89, 6), (33, 17, 72), (130, 300, 3)]
+# power-of-two z convolution; other z lengths; wide and narrow row tiles; the
+# register z convolutions on column-major spectra (FP64: lines past the last ky,
+# every block full)
+RUNTIME_MESHES = [(100, 82, 1), (40, 600, 1), (24, 1300, 1), (64, 10, 16), (97, 89, 6), (33, 17, 72), (130, 300, 3),
+                  (64, 500, 16), (32, 1024, 16), (40, 900, 16)]
 
 
 def test_run_time_passes_against_oracle(tmp_path):

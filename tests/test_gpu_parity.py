@@ -157,8 +157,9 @@ def test_column_major_3d(mesh, form):
 @pytest.mark.parametrize("mesh", [(32, 12, 16), (64, 10, 16)])
 def test_zconv_leftover_columns(mesh, form):
     """Power-of-two nx gives Hx = nx + 1 spectrum columns (33, 65): the fused z
-    convolution tiles all but the last along kx and the last along ky in the
-    same launch; field against the oracle."""
+    convolution of the run-time passes (the smaller mesh; the larger one in
+    test_run_time_passes_against_oracle) tiles all but the last along kx and the
+    last along ky in the same launch; field against the oracle."""
     from oracle.oracle import demag_tensor
 
     nx, ny, nz = mesh
@@ -508,10 +509,11 @@ def test_register_passes_fp64(mesh):
 
 @pytest.mark.parametrize("mesh", [(64, 500, 16), (32, 1024, 16)])
 def test_zquad_fp64(mesh):
-    """FP64 column-major meshes with nz = 16 (Pz = 32) run the register z
-    convolution of four threads a line: Py = 1000 (blocks past the last ky
-    line, predicated) and Py = 2048 (every block full), the shared-memory x
-    and y passes around it; H_eff and two RK4 steps against the oracle."""
+    """FP64 meshes with nz = 16 (Pz = 32) beyond the register x / y passes, on
+    compile-time lengths; H_eff and two RK4 steps against the oracle.  On the
+    run-time passes (test_run_time_passes_against_oracle, and (6, 210, 16) here by
+    default) they take the register z convolution of four threads a line: Py = 1000
+    (blocks past the last ky line, predicated) and Py = 2048 (every block full)."""
     from oracle.oracle import demag_tensor
 
     nx, ny, nz = mesh
@@ -551,8 +553,9 @@ def test_stage_tile_opt_in():
 @pytest.mark.parametrize("mesh", [(100, 60, 16), (40, 900, 16)])
 def test_zpair_layouts_fp32(mesh):
     """Pz = 32 (nz = 16) on meshes outside the register x / y passes: the
-    register-resident z convolution on row-major spectra (100 x 60) and on
-    column-major spectra (padded y = 1800): demag field against FP64."""
+    register-resident z convolution on row-major spectra between the passes on
+    compile-time lengths; demag field against FP64.  Column-major spectra
+    (padded y = 1800): test_run_time_passes_against_oracle."""
     from oracle.oracle import demag_tensor
 
     nx, ny, nz = mesh
